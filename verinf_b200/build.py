@@ -9,7 +9,7 @@ CSRC = HERE / "csrc"
 SO = HERE / "libverinf_b200.so"
 SOURCES = ["common.cu", "ntt.cu", "hash.cu", "field_ops.cu", "kquant.cu", "sumcheck.cu", "open.cu", "matmul_tc.cu", "matmul_umma.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
+              "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "--split-compile=0"]
 
 
 def _nvcc() -> str:

@@ -26,28 +26,15 @@
 #include "../../include/verinf_b200.h"
 #include "blake3.cuh"
 #include "common.cuh"
-#include "dft_reg.cuh"
-#include "gl.cuh"
+#include "dft3.cuh"
+#include "gl3.cuh"
 #include "kquant.cuh"
-#include "ntt_lanes.cuh"
-
-// Lane-form variants of the tile passes (k_pass_q, k_encode_mid_q; arithmetic of gl_lanes.cuh) are
-// compiled in only with -DVI_LANES=1.  They are bit-identical and execute 16-17 % fewer
-// instructions, spread over both integer pipes, but hold 64 data registers per thread, run at 16
-// warps per SM and came out 11-18 % slower than the 64-bit kernels on B200 (pass 1 / middle / pass 3 of
-// a 4096 x 2^16 -> 2^18 encode: 2.31 / 12.1 / 6.68 ms against 2.04 / 10.25 / 5.99 ms), so the default
-// build leaves them out.
-#ifndef VI_LANES
-#define VI_LANES 0
-#endif
 
 namespace {
 
-using vgl::add;
-using vgl::mul;
-using vgl::sub;
 using vdft::brev;
-using vdft::dif;
+using vg3::canon;
+using vg3::mul;      // any 64-bit words in, [0, 2^64) out: only what leaves the library is brought below p
 
 // Stage schedule of a length-2^LOGL tile DFT: radix-16 stages plus one smaller
 // stage (first or last).  A thread owns EPT elements of one column.
@@ -93,6 +80,8 @@ __device__ __forceinline__ uint64_t tw_at(const uint64_t* __restrict__ tw, uint3
 // pre-multiplied by w_{RHO0*L}^(t*l) except for the factor common to a thread's first butterfly,
 // w_{RHO0*L}^(t*qp), which is folded into the stage-0 twiddle here: w_L^(qp*c) * w_{RHO0*L}^(t*qp)
 // = tw0[qp*(RHO0*c + t)] with tw0 the table of w_{RHO0*L}.
+// In that case the stage-0 butterflies are the caller's as well: v comes in behind them.
+// Values are anywhere in [0, 2^64) throughout.
 template <int LOGL, bool INV, bool SMALL_LAST, int S, int RHO0 = 0>
 __device__ __forceinline__ void run_stages(uint64_t (&v)[Sched<LOGL, SMALL_LAST>::EPT], uint64_t* sm,
                                            int CP, int col, int w, const uint64_t* __restrict__ twL,
@@ -109,8 +98,10 @@ __device__ __forceinline__ void run_stages(uint64_t (&v)[Sched<LOGL, SMALL_LAST>
                 for (int i = 0; i < R; ++i)
                     v[g * R + i] = sm[((w + g * SC::TPC) + i * (L / R)) * CP + col];
         }
+        if constexpr (S > 0 || RHO0 == 0) {
 #pragma unroll
-        for (int g = 0; g < G; ++g) dif<LOGR, LOGR, INV>(&v[g * R]);
+            for (int g = 0; g < G; ++g) vd3::dif<LOGR, INV>(&v[g * R]);
+        }
         if constexpr (!LAST) {
 #pragma unroll
             for (int g = 0; g < G; ++g) {
@@ -181,27 +172,18 @@ struct PassArgs {
     const void* kq_sT;       //   and the scales per (sub-block of k, n); null = decode from the super-blocks
     uint64_t kq_magic;       // floor(2^64 / kq_dout) + 1 when the matrix has fewer than 2^32 elements (then
                              // f / kq_dout = umul64hi(f, kq_magic) exactly), else 0: 64-bit division
-    // lane-form passes (k_pass_q): the same tables as balanced 24-bit digits, and the scale likewise
-    const vln::W3* twL3;
-    const vln::W3* fs3;
-    vln::W3 scale3;
 };
 
 // Minimum resident CTAs per SM asked of the compiler for the 256-thread tiles (register budget =
-// 65536 / (256 * blocks)).  Measured on B200 at K = 2^16: k_pass 1/3/4/5/6/8 blocks -> commit
-// 32.6 / 30.2 / 27.5 / 27.3 / 28.5 / 32.0 ms; k_encode_mid is best at 2 (128 registers).
+// 65536 / (256 * blocks)).  The passes are bound by instruction issue and hold 48 data registers in a radix-16
+// butterfly: 4 blocks (64 registers) against 5 take the last pass of K = 2^14 / N = 2^16 rows from 1.90 to 1.66 ms
+// (5504 rows), and 3 blocks bring nothing (1.90); the middle pass is best at 2 (128 registers).
 #ifndef VI_PASS_MINB
-#define VI_PASS_MINB 5
+#define VI_PASS_MINB 4
 #endif
-#ifndef VI_PASS_MINB_L8
-#define VI_PASS_MINB_L8 4    // MODE 1 passes of 256-point tiles (encode pass 3 at K = 2^16: 3/4/5/6 blocks ->
-#endif                       // 6.03 / 5.98 / 6.21 / 6.56 ms; 128-point tiles prefer 5)
 #ifndef VI_MID_MINB
 #define VI_MID_MINB 2
 #endif
-#ifndef VI_PASS0_MINB
-#define VI_PASS0_MINB 4      // MODE 0 passes (strided loads straight into registers; encode pass 1 at
-#endif                       // K = 2^16: 3/4/5/6/8 blocks -> 2.95 / 2.79 / 2.89 / 3.77 / 5.11 ms)
 // Columns per tile: fixed by the tile length from 128 points up (so that all tile index arithmetic is
 // compile-time), chosen by the host from the column count below that (tile_logC on the host).
 __host__ __device__ constexpr int fixed_logC(int logl) { return logl < 7 ? -1 : logl == 7 ? 5 : logl <= 9 ? 4 : 13 - logl; }
@@ -215,7 +197,7 @@ __host__ __device__ constexpr int tile_max_threads(int logl) { return (logl >= 4
 // factor taken from two small tables (the first pass of a three-pass transform, whose full factor table
 // would have n entries)
 template <int LOGL, bool INV, int MODE, int LD = 0>
-__global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 8) ? (MODE == 0 ? VI_PASS0_MINB : (LOGL == 8 ? VI_PASS_MINB_L8 : VI_PASS_MINB)) : 1) k_pass(PassArgs a) {
+__global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 8) ? VI_PASS_MINB : 1) k_pass(PassArgs a) {
     using SC = Sched<LOGL, false>;
     constexpr int L = 1 << LOGL, EPT = SC::EPT;
     extern __shared__ uint64_t sm[];
@@ -333,8 +315,9 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
             }
         } else if constexpr (MODE == 0) {
             if (valid) v[j] = mul(v[j], __ldg(a.fs + col0 + (k * ncols32 + (uint32_t)col)));
-        } else if constexpr (INV) {
-            if (a.scale != 1) v[j] = mul(v[j], a.scale);
+        } else {
+            // this is the transform's result: the one place where it has to be canonical
+            v[j] = canon(INV ? mul(v[j], a.scale) : v[j]);
         }
     }
     if (MODE == 0 || !a.out_via_smem) {
@@ -352,113 +335,6 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
         uint64_t* dst = a.out + item * a.out_item + col0 * (int64_t)a.out_col;
         for (int e = tid; e < L * C; e += nthr) {
             int k = e & (L - 1), cl = e >> LOGL;
-            if (cl < ncols_tile) dst[(uint32_t)cl * a.out_col + (uint32_t)k * a.out_k] = sm[k * CP + cl];
-        }
-    }
-}
-
-// Resident CTAs asked of the compiler for the lane-form passes (16-byte tile elements: 3 tiles of
-// 4096 elements fit in shared memory; 64 data registers per thread).
-#ifndef VI_PASSQ_MINB
-#define VI_PASSQ_MINB 2
-#endif
-#ifndef VI_MIDQ_MINB
-#define VI_MIDQ_MINB 2
-#endif
-
-// The tile pass of k_pass in lane form (gl_lanes.cuh), for the plain loaders (LD = 0): values are
-// converted from the canonical 64-bit form as they are loaded and back as they are stored; the
-// stages in between (butterflies, stage twiddles, four-step factor, n^-1) never leave lane form.
-template <int LOGL, bool INV, int MODE>
-__global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 8) ? VI_PASSQ_MINB : 1) k_pass_q(PassArgs a) {
-    using SC = Sched<LOGL, false>;
-    using vln::Q;
-    constexpr int L = 1 << LOGL, EPT = SC::EPT;
-    extern __shared__ int4 smq[];
-    const int logC = fixed_logC(LOGL) >= 0 ? fixed_logC(LOGL) : a.logC;
-    const int tid = threadIdx.x, C = 1 << logC, CP = C + 1;
-    const int col = tid & (C - 1), w = tid >> logC;
-    const uint32_t tpi = (uint32_t)a.tiles_per_item;
-    const uint32_t item32 = blockIdx.x / tpi;
-    const int64_t item = item32;
-    const int64_t col0 = (int64_t)(blockIdx.x - item32 * tpi) * C;
-    const int64_t colg = col0 + col;
-    const bool valid = colg < a.ncols;
-    const int ncols_tile = a.ncols - col0 < C ? (int)(a.ncols - col0) : C;
-    const uint32_t ncols32 = (uint32_t)a.ncols;
-    Q v[EPT];
-    if constexpr (MODE == 0) {
-        if (a.src_kind == SRC_PLAIN) {
-            const uint64_t* src = a.in + item * a.in_item + colg * (int64_t)a.in_col;
-#pragma unroll
-            for (int j = 0; j < EPT; ++j)
-                v[j] = vln::from_u64(valid ? src[(uint32_t)SC::first_pos(j, w) * a.in_idx] : 0);
-        } else {       // message rows, zero past ELL
-            const uint64_t* src = a.in + item * a.ell;
-#pragma unroll
-            for (int j = 0; j < EPT; ++j) {
-                const int64_t slot = (int64_t)SC::first_pos(j, w) * a.in_idx + colg;
-                v[j] = vln::from_u64((valid && slot < a.ell) ? src[slot] : 0);
-            }
-        }
-    } else {
-        const int nthr = blockDim.x;
-        const uint64_t* src = a.in + item * a.in_item + col0 * (int64_t)a.in_col;
-        if (LOGL >= 4 && logC == 4) {
-            // 16 columns: the block has L threads, thread tid loads index tid of every column
-            const uint64_t* p = src + (uint32_t)tid * a.in_idx;
-            if (ncols_tile == 16) {
-#pragma unroll
-                for (int cl = 0; cl < 16; ++cl) vlt::sts_q(smq, tid * 17 + cl, vln::from_u64(p[(uint32_t)cl * a.in_col]));
-            } else {
-#pragma unroll
-                for (int cl = 0; cl < 16; ++cl)
-                    vlt::sts_q(smq, tid * 17 + cl, vln::from_u64(cl < ncols_tile ? p[(uint32_t)cl * a.in_col] : 0));
-            }
-        } else {
-            for (int e = tid; e < L * C; e += nthr) {
-                const int idx = e & (L - 1), cl = e >> LOGL;
-                vlt::sts_q(smq, idx * CP + cl,
-                           vln::from_u64(cl < ncols_tile ? src[(uint32_t)cl * a.in_col + (uint32_t)idx * a.in_idx] : 0));
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) v[j] = vlt::lds_q(smq, SC::first_pos(j, w) * CP + col);
-    }
-
-    vlt::run_stages_q<SC, LOGL, INV, 0>(v, smq, CP, col, w, a.twL3);
-
-    uint64_t o[EPT];
-#pragma unroll
-    for (int j = 0; j < EPT; ++j) {
-        const uint32_t k = SC::last_k(j, w);
-        if constexpr (MODE == 0) {
-            // first step of a four-step transform: four-step factor (also for invalid columns: any entry)
-            const vln::W3 f = vlt::ldg_w3(a.fs3 + (valid ? col0 + (k * ncols32 + (uint32_t)col) : 0));
-            o[j] = vln::to_u64(vln::mul(v[j], f));
-        } else if constexpr (INV) {
-            o[j] = vln::to_u64(vln::mul(v[j], a.scale3));      // n^-1
-        } else {
-            o[j] = vln::to_u64(v[j]);
-        }
-    }
-    if (MODE == 0 || !a.out_via_smem) {
-        if (valid) {
-            uint64_t* dst = a.out + item * a.out_item + colg * (int64_t)a.out_col;
-#pragma unroll
-            for (int j = 0; j < EPT; ++j) dst[(uint32_t)SC::last_k(j, w) * a.out_k] = o[j];
-        }
-    } else {
-        uint64_t* sm = reinterpret_cast<uint64_t*>(smq);
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) sm[SC::last_k(j, w) * CP + col] = o[j];
-        __syncthreads();
-        const int nthr = blockDim.x;
-        uint64_t* dst = a.out + item * a.out_item + col0 * (int64_t)a.out_col;
-        for (int e = tid; e < L * C; e += nthr) {
-            const int k = e & (L - 1), cl = e >> LOGL;
             if (cl < ncols_tile) dst[(uint32_t)cl * a.out_col + (uint32_t)k * a.out_k] = sm[k * CP + cl];
         }
     }
@@ -535,29 +411,26 @@ struct MidArgs {
     const uint64_t* cscale;  // K entries: K^-1 * 7^l
     const uint64_t* twRL;    // w_{rho*L}^e, e < rho*L (stage-0 twiddles of the coset transforms)
     const uint64_t* fsN;     // N entries: fsN[kk*n1 + l2] = w_N^(l2*kk), kk = rho*m1 + t
-    // lane-form kernel (k_encode_mid_q): the same tables as balanced 24-bit digits
-    const vln::W3 *twL3, *cscale3, *twRL3, *fsN3;
-    vln::W3 k_inv3;
 };
 
-// x * 2^E mod p for a compile-time E in [0, 192) (2^96 = -1)
-template <int E>
-__device__ __forceinline__ uint64_t mul_pow2_any(uint64_t x) {
-    if constexpr (E == 0) return x;
-    else if constexpr (E < 96) return vgl::mul_pow2<E>(x);
-    else return vgl::sub(0, vgl::mul_pow2<E - 96>(x));
-}
-// v[j] = c[j] * w_{16*RHO}^(T*j), j < 16: the part of the coset twist that varies inside a thread's
-// first radix-16 butterfly; w_{16*RHO} is a power of two for RHO <= 4, so these are shifts.
+// t[j] = c[j] * w_{16*RHO}^(T*j), j < 16: the part of the coset twist that varies inside a thread's
+// first radix-16 butterfly; w_{16*RHO} is a power of two for RHO <= 4, so these are shifts, and their
+// three-limb results go into the butterflies as they are.
 // The coefficients are read from the thread's own column of a shared-memory array (c[J * stride]): holding
 // them in registers across the cosets costs 32 registers and one resident CTA.
 template <int RHO, int T, int J = 0>
-__device__ __forceinline__ void coset_shift(const uint64_t* __restrict__ c, int stride, uint64_t (&v)[16]) {
+__device__ __forceinline__ void coset_shift(const uint64_t* __restrict__ c, int stride, vg3::T3 (&t)[16]) {
     if constexpr (J < 16) {
         constexpr int E = (vdft::root_exp(RHO == 4 ? 6 : RHO == 2 ? 5 : 4) * T * J) % 192;
-        v[J] = mul_pow2_any<E>(c[J * stride]);
-        coset_shift<RHO, T, J + 1>(c, stride, v);
+        t[J] = vg3::shl3<E>(vg3::widen(c[J * stride]));
+        coset_shift<RHO, T, J + 1>(c, stride, t);
     }
+}
+template <int RHO, int T>
+__device__ __forceinline__ void coset_first(const uint64_t* __restrict__ c, int stride, uint64_t (&v)[16]) {
+    vg3::T3 t[16];
+    coset_shift<RHO, T>(c, stride, t);
+    vd3::dif<4, false>(t, v);
 }
 
 // RHO = 0: any blow-up factor, twist read from the (rho, K) table (one full multiply per element
@@ -617,7 +490,7 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
     if (a.polys && valid) {
         uint64_t* dst = a.polys + item * a.K + colg;
 #pragma unroll
-        for (int j = 0; j < EPT; ++j) dst[(uint32_t)SI::last_k(j, w) * n1] = RHO == 0 ? c[j] : mul(c[j], a.k_inv);
+        for (int j = 0; j < EPT; ++j) dst[(uint32_t)SI::last_k(j, w) * n1] = canon(RHO == 0 ? c[j] : mul(c[j], a.k_inv));
     }
     if (!a.s2) return;
     uint64_t* dst2 = a.s2 + item * a.K * a.rho + colg;
@@ -657,10 +530,10 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
         for (int t = 0; t < RHO; ++t) {
             if (SF::NS > 1) __syncthreads();   // previous coset finished reading the tile
             switch (t) {
-                case 0: coset_shift<RHO, 0>(c2, nthr, v); break;
-                case 1: coset_shift<RHO, 1>(c2, nthr, v); break;
-                case 2: coset_shift<RHO, 2 % RHO>(c2, nthr, v); break;
-                default: coset_shift<RHO, 3 % RHO>(c2, nthr, v); break;
+                case 0: coset_first<RHO, 0>(c2, nthr, v); break;
+                case 1: coset_first<RHO, 1>(c2, nthr, v); break;
+                case 2: coset_first<RHO, 2 % RHO>(c2, nthr, v); break;
+                default: coset_first<RHO, 3 % RHO>(c2, nthr, v); break;
             }
             run_stages<LOGL, false, true, 0, RHO>(v, sm, CP, col, w, a.twL, a.twRL, t);
             if (valid) {
@@ -676,88 +549,6 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
     }
 }
 
-// v[j] = c[j] * w_{16*RHO}^(T*j) in lane form (lane rotations and at most one lane shift each)
-template <int RHO, int T, int J = 0>
-__device__ __forceinline__ void coset_shift_q(const uint64_t (&c)[16], vln::Q (&v)[16]) {
-    if constexpr (J < 16) {
-        constexpr int E = (vdft::root_exp(RHO == 4 ? 6 : RHO == 2 ? 5 : 4) * T * J) % 192;
-        v[J] = vln::mul_pow2<E>(vln::from_u64(c[J]));
-        coset_shift_q<RHO, T, J + 1>(c, v);
-    }
-}
-
-// The shift-twist middle pass (k_encode_mid<LOGL, RHO>, RHO = 2 or 4) in lane form, for tile lengths
-// from 128 points (every tile is full).  The scaled coefficients are kept between the cosets in
-// canonical 64-bit form (32 registers instead of 64) and unpacked per coset.
-template <int LOGL, int RHO>
-__global__ void __launch_bounds__(tile_max_threads(LOGL), LOGL <= 8 ? VI_MIDQ_MINB : 1) k_encode_mid_q(MidArgs a) {
-    using SI = Sched<LOGL, false>;   // inverse: small stage first, radix-16 last
-    using SF = Sched<LOGL, true>;    // forward: radix-16 first, small stage last
-    using vln::Q;
-    constexpr int L = 1 << LOGL, EPT = SI::EPT;
-    constexpr int LR = SI::logr(SI::NS - 1);   // last inverse radix == first forward radix
-    static_assert(LOGL >= 7 && (RHO == 2 || RHO == 4) && EPT == 16, "lane-form middle pass: full 16-column tiles");
-    extern __shared__ int4 smq[];
-    constexpr int logC = fixed_logC(LOGL), C = 1 << logC, CP = C + 1;
-    const int tid = threadIdx.x;
-    const int col = tid & (C - 1), w = tid >> logC;
-    const uint32_t tpi = (uint32_t)a.tiles_per_item;
-    const uint32_t item32 = blockIdx.x / tpi;
-    const int64_t item = item32;
-    const int64_t col0 = (int64_t)(blockIdx.x - item32 * tpi) * C;
-    const int64_t colg = col0 + col;
-    const uint32_t n1 = (uint32_t)a.n1;
-    {
-        const int nthr = blockDim.x;
-        const uint64_t* src = a.s1 + item * a.K + col0 * L;
-        if (logC == 4) {
-#pragma unroll
-            for (int cl = 0; cl < 16; ++cl) vlt::sts_q(smq, tid * 17 + cl, vln::from_u64(src[cl * L + tid]));
-        } else {
-            for (int e = tid; e < L * C; e += nthr) {
-                const int idx = e & (L - 1), cl = e >> LOGL;
-                vlt::sts_q(smq, idx * CP + cl, vln::from_u64(src[(uint32_t)(cl * L + idx)]));
-            }
-        }
-        __syncthreads();
-    }
-    Q v[EPT];
-#pragma unroll
-    for (int j = 0; j < EPT; ++j) v[j] = vlt::lds_q(smq, SI::first_pos(j, w) * CP + col);
-    vlt::run_stages_q<SI, LOGL, true, 0>(v, smq, CP, col, w, a.twL3);
-    if (a.polys) {
-        uint64_t* dst = a.polys + item * a.K + colg;
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) dst[(uint32_t)SI::last_k(j, w) * n1] = vln::to_u64(vln::mul(v[j], a.k_inv3));
-    }
-    if (!a.s2) return;
-    uint64_t* dst2 = a.s2 + item * a.K * a.rho + colg;
-    // c2[j] = coefficient l1 = first_pos(j) (held in v[brev(j)]) times K^-1 7^l, l = l1*n1 + l2
-    uint64_t c2[EPT];
-#pragma unroll
-    for (int j = 0; j < EPT; ++j) {
-        const uint32_t l1 = SF::first_pos(j, w);
-        c2[j] = vln::to_u64(vln::mul(v[brev(j, LR)], vlt::ldg_w3(a.cscale3 + colg + n1 * l1)));
-    }
-#pragma unroll 1
-    for (int t = 0; t < RHO; ++t) {
-        __syncthreads();   // previous coset (or the inverse transform) finished reading the tile
-        switch (t) {
-            case 0: coset_shift_q<RHO, 0>(c2, v); break;
-            case 1: coset_shift_q<RHO, 1>(c2, v); break;
-            case 2: coset_shift_q<RHO, 2 % RHO>(c2, v); break;
-            default: coset_shift_q<RHO, 3 % RHO>(c2, v); break;
-        }
-        vlt::run_stages_q<SF, LOGL, false, 0, RHO>(v, smq, CP, col, w, a.twL3, a.twRL3, t);
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) {
-            const uint32_t m1 = SF::last_k(j, w);
-            const uint32_t kk = m1 * RHO + (uint32_t)t;
-            dst2[kk * n1] = vln::to_u64(vln::mul(v[j], vlt::ldg_w3(a.fsN3 + colg + kk * n1)));
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Host side: twiddle cache, launch planning.
 // ---------------------------------------------------------------------------
@@ -766,7 +557,6 @@ struct DevTables {
     std::map<std::pair<int64_t, int64_t>, uint64_t*> twist;   // (K, N) -> (rho, K)
     std::map<int64_t, uint64_t*> cscale;                      // K -> K^-1 * 7^l
     std::map<std::tuple<int64_t, int64_t, bool>, uint64_t*> fs;   // (n, ncols, inverse) -> four-step factors
-    std::map<const uint64_t*, vln::W3*> w3;                   // table -> the same constants as balanced 24-bit digits
     std::map<std::pair<int64_t, bool>, std::pair<uint64_t*, uint64_t*>> split;   // (n, inverse) -> (w^e, e < 8192; w^(8192 e))
 };
 std::mutex g_mu;
@@ -790,31 +580,6 @@ int upload_table(const std::vector<uint64_t>& h, uint64_t** out) {
     return VI_OK;
 }
 
-// The lane-form kernels read their constants as three balanced 24-bit digits (vln::W3, 16 bytes).
-int upload_w3(const std::vector<uint64_t>& h, vln::W3** out) {
-    std::vector<vln::W3> hw(h.size());
-    for (size_t i = 0; i < h.size(); ++i) hw[i] = vln::make_w3(h[i]);
-    vln::W3* d = nullptr;
-    VI_CUDA(cudaMalloc(&d, hw.size() * sizeof(vln::W3)));
-    cudaError_t e = cudaMemcpy(d, hw.data(), hw.size() * sizeof(vln::W3), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e != cudaSuccess) {
-        cudaFree(d);
-        return vi::fail(VI_ERR_CUDA, "twiddle table upload: %s", cudaGetErrorString(e));
-    }
-    *out = d;
-    return VI_OK;
-}
-// digits table of a u64 table returned by get_tw / get_fs (null if there is none)
-const vln::W3* w3_of(const uint64_t* table) {
-    int dev;
-    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-    std::lock_guard<std::mutex> lk(g_mu);
-    auto& T = g_tables[dev];
-    auto it = T.w3.find(table);
-    return it == T.w3.end() ? nullptr : it->second;
-}
-
 int get_tw(int64_t n, const uint64_t** out) {
     int dev;
     VI_CUDA(cudaGetDevice(&dev));
@@ -828,13 +593,7 @@ int get_tw(int64_t n, const uint64_t** out) {
     uint64_t* d = nullptr;
     int rc_up = upload_table(h, &d);
     if (rc_up) return rc_up;
-    vln::W3* d3 = nullptr;
-#if VI_LANES
-    rc_up = upload_w3(h, &d3);
-    if (rc_up) { cudaFree(d); return rc_up; }
-#endif
     T.tw[n] = d;
-    if (d3) T.w3[d] = d3;
     *out = d;
     return VI_OK;
 }
@@ -862,13 +621,7 @@ int get_fs(int64_t n, int64_t ncols, bool inv, const uint64_t** out) {
     uint64_t* d = nullptr;
     int rc_up = upload_table(h, &d);
     if (rc_up) return rc_up;
-    vln::W3* d3 = nullptr;
-#if VI_LANES
-    rc_up = upload_w3(h, &d3);
-    if (rc_up) { cudaFree(d); return rc_up; }
-#endif
     T.fs[key] = d;
-    if (d3) T.w3[d] = d3;
     *out = d;
     return VI_OK;
 }
@@ -937,13 +690,7 @@ int get_cscale(int64_t K, const uint64_t** out) {
     uint64_t* d = nullptr;
     int rc_up = upload_table(h, &d);
     if (rc_up) return rc_up;
-    vln::W3* d3 = nullptr;
-#if VI_LANES
-    rc_up = upload_w3(h, &d3);
-    if (rc_up) { cudaFree(d); return rc_up; }
-#endif
     T.cscale[K] = d;
-    if (d3) T.w3[d] = d3;
     *out = d;
     return VI_OK;
 }
@@ -968,25 +715,8 @@ int tile_threads(int logL, int logC) {
 }
 size_t tile_smem(int logL, int logC) { return (size_t)(1 << logL) * ((1 << logC) + 1) * 8; }
 
-template <int LOGL, bool INV, int MODE>
-int launch_pass_q(const PassArgs& a, int64_t items, cudaStream_t st, int tag) {
-    size_t smem = 2 * tile_smem(LOGL, a.logC);
-    auto fn = k_pass_q<LOGL, INV, MODE>;
-    if (smem > 48 * 1024) VI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int64_t grid = items * a.tiles_per_item;
-    if (grid <= 0) return VI_OK;
-    if (grid > 0x7FFFFFFFLL) return vi::fail(VI_ERR_LIMIT, "tile grid too large (%lld)", (long long)grid);
-    vi::ProfScope prof(tag, st);
-    fn<<<(unsigned)grid, tile_threads(LOGL, a.logC), smem, st>>>(a);
-    return vi::check_launch("k_pass_q");
-}
-
 template <int LOGL, bool INV, int MODE, int LD = 0>
 int launch_pass_t(const PassArgs& a, int64_t items, cudaStream_t st, int tag) {
-    if constexpr (VI_LANES && LD == 0 && LOGL >= 4 && LOGL <= 10) {
-        if (a.twL3 != nullptr && (MODE == 1 || a.fs3 != nullptr) && (a.src_kind == SRC_PLAIN || a.src_kind == SRC_MSG))
-            return launch_pass_q<LOGL, INV, MODE>(a, items, st, tag);
-    }
     size_t smem = tile_smem(LOGL, a.logC);
     auto fn = k_pass<LOGL, INV, MODE, LD>;
     if (smem > 48 * 1024) VI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1041,9 +771,6 @@ int launch_pass(int logL, bool inv, int mode, PassArgs& a, int64_t items, cudaSt
     a.tiles_per_item = (a.ncols + (1 << a.logC) - 1) >> a.logC;
     int rc = get_tw(int64_t(1) << logL, &a.twL);
     if (rc) return rc;
-    a.twL3 = w3_of(a.twL);
-    a.fs3 = (a.fs && !a.fs_hi) ? w3_of(a.fs) : nullptr;
-    a.scale3 = vln::make_w3(a.scale);
     if (inv) return mode ? launch_pass_l<true, 1>(logL, a, items, st, tag) : launch_pass_l<true, 0>(logL, a, items, st, tag);
     return mode ? launch_pass_l<false, 1>(logL, a, items, st, tag) : launch_pass_l<false, 0>(logL, a, items, st, tag);
 }
@@ -1065,28 +792,7 @@ int launch_mid_t(const MidArgs& a, int64_t items, cudaStream_t st) {
 bool mid_shift_form(int logL, int64_t rho) {
     return (rho == 2 || rho == 4) && logL >= 4 && logL <= 10;
 }
-template <int LOGL, int RHO>
-int launch_mid_q(const MidArgs& a, int64_t items, cudaStream_t st) {
-    size_t smem = 2 * tile_smem(LOGL, a.logC);
-    auto fn = k_encode_mid_q<LOGL, RHO>;
-    if (smem > 48 * 1024) VI_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int64_t grid = items * a.tiles_per_item;
-    if (grid <= 0) return VI_OK;
-    if (grid > 0x7FFFFFFFLL) return vi::fail(VI_ERR_LIMIT, "tile grid too large (%lld)", (long long)grid);
-    vi::ProfScope prof(vi::PROF_ENC_MID, st);
-    fn<<<(unsigned)grid, tile_threads(LOGL, a.logC), smem, st>>>(a);
-    return vi::check_launch("k_encode_mid_q");
-}
 int launch_mid(int logL, const MidArgs& a, int64_t items, cudaStream_t st) {
-#if VI_LANES
-    if (mid_shift_form(logL, a.rho) && logL >= 7 && a.twL3 && a.cscale3 && a.twRL3 && a.fsN3) {
-        switch (logL * 8 + a.rho) {
-#define VI_CASE(x) case x * 8 + 2: return launch_mid_q<x, 2>(a, items, st); case x * 8 + 4: return launch_mid_q<x, 4>(a, items, st);
-            VI_CASE(7) VI_CASE(8) VI_CASE(9) VI_CASE(10)
-#undef VI_CASE
-        }
-    }
-#endif
     if (mid_shift_form(logL, a.rho)) {
         switch (logL * 8 + a.rho) {
 #define VI_CASE(x) case x * 8 + 2: return launch_mid_t<x, 2>(a, items, st); case x * 8 + 4: return launch_mid_t<x, 4>(a, items, st);
@@ -1130,7 +836,6 @@ extern "C" int vi_release_tables(void) {
         for (auto& t : kv.second.twist) cudaFree(t.second);
         for (auto& t : kv.second.fs) cudaFree(t.second);
         for (auto& t : kv.second.cscale) cudaFree(t.second);
-        for (auto& t : kv.second.w3) cudaFree(t.second);
         for (auto& t : kv.second.split) { cudaFree(t.second.first); cudaFree(t.second.second); }
     }
     g_tables.clear();
@@ -1392,11 +1097,6 @@ static int encode_impl(const uint64_t* msg, const KqSrc* kq, int64_t m, int64_t 
         mid.cscale = cscale; mid.twRL = twRL; mid.fsN = fsN;
         rc = get_tw(n2, &mid.twL);
         if (rc) return rc;
-        mid.twL3 = w3_of(mid.twL);
-        mid.cscale3 = cscale ? w3_of(cscale) : nullptr;
-        mid.twRL3 = twRL ? w3_of(twRL) : nullptr;
-        mid.fsN3 = fsN ? w3_of(fsN) : nullptr;
-        mid.k_inv3 = vln::make_w3(mid.k_inv);
         rc = launch_mid(log2, mid, cnt, st);
         if (rc) return rc;
         if (!codes) continue;
