@@ -55,37 +55,41 @@ struct Sched {
         for (int i = 0; i < s; ++i) p += logr(i);
         return p;
     }
-    // register j of the first stage holds input index first_pos(j, w)
-    __host__ __device__ static constexpr int first_pos(int j, int w) {
+    // register j of the first stage of thread w holds input index w + first_off(j).  (Indices are split that way
+    // everywhere: the thread's part is multiplied by a stride once, the rest is the same for all threads.)
+    __host__ __device__ static constexpr int first_off(int j) {
         if (NS == 0) return 0;
         int r = 1 << logr(0);
-        return (w + (j / r) * TPC) + (j % r) * ((1 << LOGL) / r);
+        return (j / r) * TPC + (j % r) * ((1 << LOGL) / r);
     }
-    // register j after the last stage holds output index last_k(j, w)
-    __host__ __device__ static constexpr int last_k(int j, int w) {
+    // register j after the last stage holds output index w + last_off(j)
+    __host__ __device__ static constexpr int last_off(int j) {
         if (NS == 0) return 0;
         int lr = logr(NS - 1), r = 1 << lr;
-        return (w + (j / r) * TPC) + brev(j % r, lr) * ((1 << LOGL) / r);
+        return (j / r) * TPC + brev(j % r, lr) * ((1 << LOGL) / r);
+    }
+    // Twiddles of the stages, in the order in which threads read them: stage s at stage_tw(s), entry
+    // [c][qp] = w_L^(+-(qp*c) << logp(s)) for output digit c and qp < L >> (logp(s) + logr(s)), so that a thread's loads
+    // are one address and compile-time offsets.  With a coset form of RHO0 cosets, stage 0 holds RHO0 such blocks
+    // (see run_stages).
+    __host__ __device__ static constexpr int stage_tw(int s, int rho0 = 0) {
+        int o = 0;
+        for (int i = 0; i < s; ++i) o += ((1 << LOGL) >> logp(i)) * (i == 0 && rho0 ? rho0 : 1);
+        return o;
     }
 };
 
-template <bool INV>
-__device__ __forceinline__ uint64_t tw_at(const uint64_t* __restrict__ tw, uint32_t e, uint32_t mask) {
-    return INV ? __ldg(tw + ((0u - e) & mask)) : __ldg(tw + e);   // w^-e = w^(n-e)
-}
-
 // Stages S..NS-1 of the tile DFT.  v is preloaded for stage S; on return it holds
-// the outputs of the last stage (see Sched::last_k).  sm is the tile [pos*CP + col].
+// the outputs of the last stage (see Sched::last_off).  sm is the tile [pos*CP + col].
 // RHO0 > 0 (forward only): the transform is the coset t of a length RHO0*L transform, input
 // pre-multiplied by w_{RHO0*L}^(t*l) except for the factor common to a thread's first butterfly,
 // w_{RHO0*L}^(t*qp), which is folded into the stage-0 twiddle here: w_L^(qp*c) * w_{RHO0*L}^(t*qp)
-// = tw0[qp*(RHO0*c + t)] with tw0 the table of w_{RHO0*L}.
+// = w_{RHO0*L}^(qp*(RHO0*c + t)), block t of stage 0 in the table.
 // In that case the stage-0 butterflies are the caller's as well: v comes in behind them.
 // Values are anywhere in [0, 2^64) throughout.
 template <int LOGL, bool INV, bool SMALL_LAST, int S, int RHO0 = 0>
 __device__ __forceinline__ void run_stages(uint64_t (&v)[Sched<LOGL, SMALL_LAST>::EPT], uint64_t* sm,
-                                           int CP, int col, int w, const uint64_t* __restrict__ twL,
-                                           const uint64_t* __restrict__ tw0 = nullptr, int t = 0) {
+                                           int CP, int col, int w, const uint64_t* __restrict__ tw, int t = 0) {
     using SC = Sched<LOGL, SMALL_LAST>;
     if constexpr (S < SC::NS) {
         constexpr int LOGR = SC::logr(S), R = 1 << LOGR, G = SC::EPT / R, LOGP = SC::logp(S);
@@ -105,19 +109,13 @@ __device__ __forceinline__ void run_stages(uint64_t (&v)[Sched<LOGL, SMALL_LAST>
         if constexpr (!LAST) {
 #pragma unroll
             for (int g = 0; g < G; ++g) {
-                uint32_t qp = (uint32_t)(w + g * SC::TPC) >> LOGP;
-                if constexpr (S == 0 && RHO0 > 0) {
-                    static_assert(!INV && LOGP == 0, "coset twiddles: forward stage 0 only");
+                constexpr int NQ = L >> (LOGP + LOGR);
+                constexpr bool COSET = S == 0 && RHO0 > 0;
+                static_assert(!COSET || (!INV && LOGP == 0), "coset twiddles: forward stage 0 only");
+                const uint64_t* twp = tw + SC::stage_tw(S, RHO0) + (COSET ? t * L : 0) + ((w + g * SC::TPC) >> LOGP);
 #pragma unroll
-                    for (int c = 0; c < R; ++c)
-                        v[g * R + brev(c, LOGR)] = mul(v[g * R + brev(c, LOGR)], __ldg(tw0 + qp * (uint32_t)(RHO0 * c + t)));
-                } else {
-#pragma unroll
-                    for (int c = 1; c < R; ++c) {
-                        uint32_t e = (qp * c) << LOGP;
-                        v[g * R + brev(c, LOGR)] = mul(v[g * R + brev(c, LOGR)], tw_at<INV>(twL, e, L - 1));
-                    }
-                }
+                for (int c = COSET ? 0 : 1; c < R; ++c)
+                    v[g * R + brev(c, LOGR)] = mul(v[g * R + brev(c, LOGR)], __ldg(twp + c * NQ));
             }
             __syncthreads();
 #pragma unroll
@@ -129,7 +127,7 @@ __device__ __forceinline__ void run_stages(uint64_t (&v)[Sched<LOGL, SMALL_LAST>
                     sm[(qp * PP * R + kappa + PP * c) * CP + col] = v[g * R + brev(c, LOGR)];
             }
             __syncthreads();
-            run_stages<LOGL, INV, SMALL_LAST, S + 1, RHO0>(v, sm, CP, col, w, twL, tw0, t);
+            run_stages<LOGL, INV, SMALL_LAST, S + 1, RHO0>(v, sm, CP, col, w, tw, t);
         }
     }
 }
@@ -146,9 +144,9 @@ struct PassArgs {
     int64_t ncols;           // columns per item
     int64_t tiles_per_item;
     int64_t in_item, out_item;        // element stride between items (64-bit)
-    uint32_t in_idx, in_col;          // element strides inside a tile (32-bit offsets from the tile base)
+    uint32_t in_idx;                  // MODE 0: element stride between input indices (columns are adjacent)
     uint32_t out_k, out_col;
-    const uint64_t* twL;     // w_L^e, e < L
+    const uint64_t* tw;      // stage twiddles (Sched::stage_tw)
     const uint64_t* fs;      // four-step factors, fs[k*ncols + col] = w_n^(+-col*k), or null
     const uint64_t* fs_hi;   // split factor form (LD = 3, transforms above 2^24): w_n^(+-e) = fs[e & 8191] * fs_hi[e >> 13]
     uint64_t scale;          // multiply outputs by this unless 1
@@ -176,14 +174,13 @@ struct PassArgs {
 
 // Minimum resident CTAs per SM asked of the compiler for the 256-thread tiles (register budget =
 // 65536 / (256 * blocks)).  The passes are bound by instruction issue and hold 48 data registers in a radix-16
-// butterfly: 4 blocks (64 registers) against 5 take the last pass of K = 2^14 / N = 2^16 rows from 1.90 to 1.66 ms
-// (5504 rows), and 3 blocks bring nothing (1.90); the middle pass is best at 2 (128 registers).
-#ifndef VI_PASS_MINB
-#define VI_PASS_MINB 4
-#endif
-#ifndef VI_MID_MINB
-#define VI_MID_MINB 2
-#endif
+// butterfly.  Measured (4096 rows, K = 2^16, 2 / 3 / 4 / 5 blocks where taken): plain first pass 1.48 ms at 3, 1.55 at 4
+// (which spills 16 bytes); with the pad PRG or the K-quant lift in its loader 4 is 1-4 % better; last pass 4.59 at 3,
+// 4.11 at 4, 15 % worse at 5; middle pass 6.80 at 2, 6.65 at 3.
+constexpr int pass_min_ctas(int logl, int mode, int ld) {
+    return logl < 4 || logl > 8 ? 1 : mode == 0 && (ld == 0 || ld == 3) ? 3 : 4;
+}
+constexpr int mid_min_ctas(int logl) { return logl < 4 || logl > 8 ? 1 : 3; }
 // Columns per tile: fixed by the tile length from 128 points up (so that all tile index arithmetic is
 // compile-time), chosen by the host from the column count below that (tile_logC on the host).
 __host__ __device__ constexpr int fixed_logC(int logl) { return logl < 7 ? -1 : logl == 7 ? 5 : logl <= 9 ? 4 : 13 - logl; }
@@ -191,13 +188,36 @@ __host__ __device__ constexpr int fixed_logC(int logl) { return logl < 7 ? -1 : 
 // tiles of DFT length 2^4..2^8 always run 256 threads (4096 elements / 16 per thread)
 __host__ __device__ constexpr int tile_max_threads(int logl) { return (logl >= 4 && logl <= 8) ? 256 : 512; }
 
+// Tile of C columns that lie one after the other in memory (L values each) into shared memory, sm[idx*CP + column];
+// columns from `valid` on are zero.
+template <int LOGL>
+__device__ __forceinline__ void load_tile(uint64_t* sm, const uint64_t* __restrict__ src, int CP, int valid, int C) {
+    constexpr int L = 1 << LOGL, LC = fixed_logC(LOGL);
+    const int tid = threadIdx.x;
+    if (LC >= 0 && valid == C) {
+        // 16 values per thread, at compile-time distances on both sides
+        constexpr int NT = LC >= 0 ? (L / 16) << LC : 1, PER = L > NT ? L / NT : 1;
+        uint64_t* d = sm + (tid & (L - 1)) * CP + (L > NT ? 0 : tid >> LOGL);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            if (L > NT) d[(i % PER) * NT * CP + i / PER] = src[tid + i * NT];
+            else d[i * (NT >> LOGL)] = src[tid + i * NT];
+        }
+    } else {
+        for (int e = tid; e < L * C; e += blockDim.x) {
+            const int idx = e & (L - 1), cl = e >> LOGL;
+            sm[idx * CP + cl] = cl < valid ? src[e] : 0;
+        }
+    }
+}
+
 // LD selects the loader of a MODE 0 pass at compile time, so that the plain loaders do not carry the
 // registers, code and barrier of the others: 0 = plain rows or message rows without pad, 1 = message
 // rows with the PRG pad, 2 = K-quant lift (pad decided at run time), 3 = plain rows with the four-step
 // factor taken from two small tables (the first pass of a three-pass transform, whose full factor table
 // would have n entries)
 template <int LOGL, bool INV, int MODE, int LD = 0>
-__global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 8) ? VI_PASS_MINB : 1) k_pass(PassArgs a) {
+__global__ void __launch_bounds__(tile_max_threads(LOGL), pass_min_ctas(LOGL, MODE, LD)) k_pass(PassArgs a) {
     using SC = Sched<LOGL, false>;
     constexpr int L = 1 << LOGL, EPT = SC::EPT;
     extern __shared__ uint64_t sm[];
@@ -215,10 +235,10 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
     uint64_t v[EPT];
     if constexpr (MODE == 0) {
         if ((LD == 0 || LD == 3) && a.src_kind == SRC_PLAIN) {
-            const uint64_t* src = a.in + item * a.in_item + colg * (int64_t)a.in_col;
+            const uint64_t* src = a.in + item * a.in_item + colg + (int64_t)w * a.in_idx;
 #pragma unroll
             for (int j = 0; j < EPT; ++j)
-                v[j] = valid ? src[(uint32_t)SC::first_pos(j, w) * a.in_idx] : 0;
+                v[j] = valid ? src[(uint32_t)SC::first_off(j) * a.in_idx] : 0;
         } else {
             const uint64_t* src = a.in + item * a.ell;
             uint32_t seed[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -239,9 +259,10 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
                 }
                 __syncthreads();
             }
+            const int64_t slot0 = (int64_t)w * a.in_idx + colg;
 #pragma unroll
             for (int j = 0; j < EPT; ++j) {
-                int64_t slot = (int64_t)SC::first_pos(j, w) * a.in_idx + colg;
+                const int64_t slot = (int64_t)SC::first_off(j) * a.in_idx + slot0;
                 uint64_t x = 0;
                 if (valid) {
                     if (slot < a.ell) {
@@ -277,44 +298,27 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
             }
         }
     } else {
-        const int nthr = blockDim.x;
-        const uint64_t* src = a.in + item * a.in_item + col0 * (int64_t)a.in_col;
-        if (LOGL >= 4 && logC == 4) {
-            // 16 columns: the block has L threads, thread tid loads index tid of every column
-            const uint64_t* p = src + (uint32_t)tid * a.in_idx;
-            if (ncols_tile == 16) {
-#pragma unroll
-                for (int cl = 0; cl < 16; ++cl) sm[tid * 17 + cl] = p[(uint32_t)cl * a.in_col];
-            } else {
-#pragma unroll
-                for (int cl = 0; cl < 16; ++cl) sm[tid * 17 + cl] = cl < ncols_tile ? p[(uint32_t)cl * a.in_col] : 0;
-            }
-        } else {
-            for (int e = tid; e < L * C; e += nthr) {
-                int idx = e & (L - 1), cl = e >> LOGL;
-                sm[idx * CP + cl] = cl < ncols_tile ? src[(uint32_t)cl * a.in_col + (uint32_t)idx * a.in_idx] : 0;
-            }
-        }
+        load_tile<LOGL>(sm, a.in + item * a.in_item + col0 * L, CP, ncols_tile, C);
         __syncthreads();
 #pragma unroll
-        for (int j = 0; j < EPT; ++j) v[j] = sm[SC::first_pos(j, w) * CP + col];
+        for (int j = 0; j < EPT; ++j) v[j] = sm[(w + SC::first_off(j)) * CP + col];
     }
 
-    run_stages<LOGL, INV, false, 0>(v, sm, CP, col, w, a.twL);
+    run_stages<LOGL, INV, false, 0>(v, sm, CP, col, w, a.tw);
 
+    const uint64_t* fs = (MODE == 0 && LD != 3) ? a.fs + colg + (int64_t)w * ncols32 : nullptr;
 #pragma unroll
     // Every MODE 0 pass is the first step of a four-step transform: four-step factor, no scaling, strided
     // store.  MODE 1 passes are last steps: no factor, n^-1 on inverse transforms, and a store through
     // shared memory only for the single-pass transform (rows contiguous along the output index).
     for (int j = 0; j < EPT; ++j) {
-        uint32_t k = SC::last_k(j, w);
         if constexpr (MODE == 0 && LD == 3) {
             if (valid) {
-                const uint64_t e = (uint64_t)k * (uint64_t)colg;       // < n
+                const uint64_t e = (uint64_t)(w + SC::last_off(j)) * (uint64_t)colg;       // < n
                 v[j] = mul(mul(v[j], __ldg(a.fs + (e & 8191))), __ldg(a.fs_hi + (e >> 13)));
             }
         } else if constexpr (MODE == 0) {
-            if (valid) v[j] = mul(v[j], __ldg(a.fs + col0 + (k * ncols32 + (uint32_t)col)));
+            if (valid) v[j] = mul(v[j], __ldg(fs + (uint32_t)SC::last_off(j) * ncols32));
         } else {
             // this is the transform's result: the one place where it has to be canonical
             v[j] = canon(INV ? mul(v[j], a.scale) : v[j]);
@@ -322,20 +326,25 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
     }
     if (MODE == 0 || !a.out_via_smem) {
         if (valid) {
-            uint64_t* dst = a.out + item * a.out_item + colg * (int64_t)a.out_col;
+            uint64_t* dst = a.out + item * a.out_item + colg * (int64_t)a.out_col + (int64_t)w * a.out_k;
 #pragma unroll
-            for (int j = 0; j < EPT; ++j) dst[(uint32_t)SC::last_k(j, w) * a.out_k] = v[j];
+            for (int j = 0; j < EPT; ++j) dst[(uint32_t)SC::last_off(j) * a.out_k] = v[j];
         }
     } else {
         __syncthreads();
 #pragma unroll
-        for (int j = 0; j < EPT; ++j) sm[SC::last_k(j, w) * CP + col] = v[j];
+        for (int j = 0; j < EPT; ++j) sm[(w + SC::last_off(j)) * CP + col] = v[j];
         __syncthreads();
-        const int nthr = blockDim.x;
-        uint64_t* dst = a.out + item * a.out_item + col0 * (int64_t)a.out_col;
-        for (int e = tid; e < L * C; e += nthr) {
-            int k = e & (L - 1), cl = e >> LOGL;
-            if (cl < ncols_tile) dst[(uint32_t)cl * a.out_col + (uint32_t)k * a.out_k] = sm[k * CP + cl];
+        uint64_t* dst = a.out + item * a.out_item + col0 * L;     // rows of L values, one after the other
+        constexpr int LC = fixed_logC(LOGL);
+        if (LC >= 0 && ncols_tile == C) {
+            constexpr int NT = LC >= 0 ? (L / 16) << LC : 1, PER = L > NT ? L / NT : 1;
+            const int k0 = tid & (L - 1), c0 = L > NT ? 0 : tid >> LOGL;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                dst[tid + i * NT] = sm[(k0 + (i % PER) * NT) * CP + c0 + (L > NT ? i / PER : i * (NT >> LOGL))];
+        } else {
+            for (int e = tid; e < L * ncols_tile; e += blockDim.x) dst[e] = sm[(e & (L - 1)) * CP + (e >> LOGL)];
         }
     }
 }
@@ -403,13 +412,13 @@ struct MidArgs {
     int64_t tiles_per_item;
     int rho;
     int64_t K;
-    const uint64_t* twL;   // w_L^e
+    const uint64_t* tw_inv;  // stage twiddles of the inverse transform and of the forward ones (coset form with RHO > 0)
+    const uint64_t* tw_fwd;
     const uint64_t* fsK;   // forward four-step factors, fsK[m1*n1 + l2] = w_K^(l2*m1)
     const uint64_t* twist; // (rho, K): (7*w_N^t)^l
     uint64_t k_inv;
     // shift-twist form (RHO template parameter 2 or 4):
     const uint64_t* cscale;  // K entries: K^-1 * 7^l
-    const uint64_t* twRL;    // w_{rho*L}^e, e < rho*L (stage-0 twiddles of the coset transforms)
     const uint64_t* fsN;     // N entries: fsN[kk*n1 + l2] = w_N^(l2*kk), kk = rho*m1 + t
 };
 
@@ -439,7 +448,7 @@ __device__ __forceinline__ void coset_first(const uint64_t* __restrict__ c, int 
 // w_N^(t*l2) (folded into the four-step factor table), w_{RHO L}^(t*w) (folded into the stage-0
 // twiddle) and w_{16 RHO}^(t*j), a power of two applied as a shift: no twist multiply remains.
 template <int LOGL, int RHO>
-__global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 8) ? VI_MID_MINB : 1) k_encode_mid(MidArgs a) {
+__global__ void __launch_bounds__(tile_max_threads(LOGL), mid_min_ctas(LOGL)) k_encode_mid(MidArgs a) {
     using SI = Sched<LOGL, false>;   // inverse: small stage first, radix-16 last
     using SF = Sched<LOGL, true>;    // forward: radix-16 first, small stage last
     constexpr int L = 1 << LOGL, EPT = SI::EPT;
@@ -459,71 +468,52 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
     const int ncols_tile = fixed_logC(LOGL) >= 0 ? C : (a.n1 - col0 < C ? (int)(a.n1 - col0) : C);
     const uint32_t n1 = (uint32_t)a.n1, rho = (uint32_t)a.rho;
 
-    {
-        const int nthr = blockDim.x;
-        const uint64_t* src = a.s1 + item * a.K + col0 * L;
-        if (LOGL >= 4 && logC == 4) {
-            // 16 columns: the block has L threads, thread tid loads index tid of every column
-            if (ncols_tile == 16) {
-#pragma unroll
-                for (int cl = 0; cl < 16; ++cl) sm[tid * 17 + cl] = src[cl * L + tid];
-            } else {
-#pragma unroll
-                for (int cl = 0; cl < 16; ++cl) sm[tid * 17 + cl] = cl < ncols_tile ? src[cl * L + tid] : 0;
-            }
-        } else {
-            for (int e = tid; e < L * C; e += nthr) {
-                int idx = e & (L - 1), cl = e >> LOGL;
-                sm[idx * CP + cl] = cl < ncols_tile ? src[(uint32_t)(cl * L + idx)] : 0;
-            }
-        }
-        __syncthreads();
-    }
+    load_tile<LOGL>(sm, a.s1 + item * a.K + col0 * L, CP, ncols_tile, C);
+    __syncthreads();
     uint64_t c[EPT], v[EPT];
 #pragma unroll
-    for (int j = 0; j < EPT; ++j) c[j] = sm[SI::first_pos(j, w) * CP + col];
-    run_stages<LOGL, true, false, 0>(c, sm, CP, col, w, a.twL);
+    for (int j = 0; j < EPT; ++j) c[j] = sm[(w + SI::first_off(j)) * CP + col];
+    run_stages<LOGL, true, false, 0>(c, sm, CP, col, w, a.tw_inv);
     if constexpr (RHO == 0) {
 #pragma unroll
         for (int j = 0; j < EPT; ++j) c[j] = mul(c[j], a.k_inv);
     }
     if (a.polys && valid) {
-        uint64_t* dst = a.polys + item * a.K + colg;
+        uint64_t* dst = a.polys + item * a.K + colg + (int64_t)w * n1;
 #pragma unroll
-        for (int j = 0; j < EPT; ++j) dst[(uint32_t)SI::last_k(j, w) * n1] = canon(RHO == 0 ? c[j] : mul(c[j], a.k_inv));
+        for (int j = 0; j < EPT; ++j) dst[(uint32_t)SI::last_off(j) * n1] = canon(RHO == 0 ? c[j] : mul(c[j], a.k_inv));
     }
     if (!a.s2) return;
-    uint64_t* dst2 = a.s2 + item * a.K * a.rho + colg;
+    uint64_t* dst2 = a.s2 + item * a.K * a.rho + colg + (int64_t)w * rho * n1;
     if constexpr (RHO == 0) {
         for (int t = 0; t < a.rho; ++t) {
-            const uint64_t* tw_t = a.twist + (int64_t)t * a.K + colg;
+            const uint64_t* tw_t = a.twist + (int64_t)t * a.K + colg + (int64_t)w * n1;
             if (SF::NS > 1) __syncthreads();   // previous coset finished reading the tile
 #pragma unroll
             for (int j = 0; j < EPT; ++j) {
-                // forward register j needs coefficient index l1 = first_pos(j): it is held in c[brev(j)]
-                uint32_t l1 = SF::first_pos(j, w);
-                uint64_t tw = valid ? __ldg(tw_t + n1 * l1) : 0;
+                // forward register j needs coefficient index l1 = w + first_off(j): it is held in c[brev(j)]
+                uint64_t tw = valid ? __ldg(tw_t + n1 * (uint32_t)SF::first_off(j)) : 0;
                 v[j] = mul(c[(j / (1 << LR)) * (1 << LR) + brev(j % (1 << LR), LR)], tw);
             }
-            run_stages<LOGL, false, true, 0>(v, sm, CP, col, w, a.twL);
+            run_stages<LOGL, false, true, 0>(v, sm, CP, col, w, a.tw_fwd);
             if (valid) {
 #pragma unroll
                 for (int j = 0; j < EPT; ++j) {
-                    uint32_t m1 = SF::last_k(j, w);
-                    uint64_t x = mul(v[j], __ldg(a.fsK + colg + m1 * n1));
-                    dst2[(m1 * rho + (uint32_t)t) * n1] = x;
+                    const uint32_t m1 = SF::last_off(j);
+                    dst2[(m1 * rho + (uint32_t)t) * n1] = mul(v[j], __ldg(a.fsK + colg + (int64_t)w * n1 + m1 * n1));
                 }
             }
         }
     } else {
-        // c2[j] = coefficient l1 = first_pos(j) (held in c[brev(j)]) times K^-1 7^l, l = l1*n1 + l2; kept in
+        // c2[j] = coefficient l1 = w + first_off(j) (held in c[brev(j)]) times K^-1 7^l, l = l1*n1 + l2; kept in
         // shared memory behind the tile, element j of thread tid at c2[j * blockDim.x + tid]
         uint64_t* c2 = sm + (size_t)L * CP + tid;
         const int nthr = blockDim.x;
+        const uint64_t* cs = a.cscale + colg + (int64_t)w * n1;
+        const uint64_t* fs = a.fsN + colg + (int64_t)w * RHO * n1;
 #pragma unroll
         for (int j = 0; j < EPT; ++j) {
-            uint32_t l1 = SF::first_pos(j, w);
-            uint64_t sc = valid ? __ldg(a.cscale + colg + n1 * l1) : 0;
+            uint64_t sc = valid ? __ldg(cs + n1 * (uint32_t)SF::first_off(j)) : 0;
             c2[j * nthr] = mul(c[brev(j, LR)], sc);
         }
 #pragma unroll 1   // (fully unrolled: no spills, but 11.9 ms against 10.9 ms at K = 2^16)
@@ -535,16 +525,16 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
                 case 2: coset_first<RHO, 2 % RHO>(c2, nthr, v); break;
                 default: coset_first<RHO, 3 % RHO>(c2, nthr, v); break;
             }
-            run_stages<LOGL, false, true, 0, RHO>(v, sm, CP, col, w, a.twL, a.twRL, t);
-            if (valid) {
+            run_stages<LOGL, false, true, 0, RHO>(v, sm, CP, col, w, a.tw_fwd, t);
+            if (valid) {     // index kk = m1*RHO + t, m1 = w + last_off(j)
 #pragma unroll
                 for (int j = 0; j < EPT; ++j) {
-                    uint32_t m1 = SF::last_k(j, w);
-                    uint32_t kk = m1 * RHO + (uint32_t)t;
-                    uint64_t x = mul(v[j], __ldg(a.fsN + colg + kk * n1));
-                    dst2[kk * n1] = x;
+                    const uint32_t kk = (uint32_t)SF::last_off(j) * RHO * n1;
+                    dst2[kk] = mul(v[j], __ldg(fs + kk));
                 }
             }
+            dst2 += n1;
+            fs += n1;
         }
     }
 }
@@ -553,7 +543,7 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), (LOGL >= 4 && LOGL <= 
 // Host side: twiddle cache, launch planning.
 // ---------------------------------------------------------------------------
 struct DevTables {
-    std::map<int64_t, uint64_t*> tw;                          // n -> w_n^e, e < n
+    std::map<std::tuple<int, bool, bool, int>, uint64_t*> tw;  // (log L, small stage last, inverse, cosets) -> stage twiddles
     std::map<std::pair<int64_t, int64_t>, uint64_t*> twist;   // (K, N) -> (rho, K)
     std::map<int64_t, uint64_t*> cscale;                      // K -> K^-1 * 7^l
     std::map<std::tuple<int64_t, int64_t, bool>, uint64_t*> fs;   // (n, ncols, inverse) -> four-step factors
@@ -580,20 +570,43 @@ int upload_table(const std::vector<uint64_t>& h, uint64_t** out) {
     return VI_OK;
 }
 
-int get_tw(int64_t n, const uint64_t** out) {
+// stage twiddles of a tile DFT of length 2^logl in reading order (Sched::stage_tw); rho > 0: stage 0 holds the blocks
+// w_{rho L}^(qp*(rho*c + t)) of the cosets t < rho
+template <bool SMALL_LAST, int LOGL = 12>
+std::vector<uint64_t> stage_twiddles(int logl, bool inv, int rho) {
+    if constexpr (LOGL >= 0) {
+        if (logl != LOGL) return stage_twiddles<SMALL_LAST, LOGL - 1>(logl, inv, rho);
+        using SC = Sched<LOGL, SMALL_LAST>;
+        constexpr int64_t L = int64_t(1) << LOGL;
+        const int64_t n = L * (rho ? rho : 1);
+        uint64_t wn = vgl::hpow(7, (vgl::P - 1) / (uint64_t)n);
+        if (inv) wn = vgl::hpow(wn, vgl::P - 2);
+        std::vector<uint64_t> pw((size_t)n), h;
+        pw[0] = 1;
+        for (int64_t e = 1; e < n; ++e) pw[(size_t)e] = vgl::hmul(pw[(size_t)e - 1], wn);
+        for (int s = 0; s < SC::NS; ++s)
+            for (int t = 0; t < (s == 0 && rho ? rho : 1); ++t)
+                for (int64_t c = 0; c < (int64_t(1) << SC::logr(s)); ++c)
+                    for (int64_t qp = 0; qp < L >> (SC::logp(s) + SC::logr(s)); ++qp)
+                        h.push_back(pw[(size_t)((s == 0 && rho ? qp * (rho * c + t) : ((qp * c) << SC::logp(s)) * (rho ? rho : 1)) % n)]);
+        if (h.empty()) h.push_back(1);
+        return h;
+    } else {
+        return {};
+    }
+}
+int get_tw(int logl, bool small_last, bool inv, int rho, const uint64_t** out) {
     int dev;
     VI_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(g_mu);
     auto& T = g_tables[dev];
-    auto it = T.tw.find(n);
+    auto key = std::make_tuple(logl, small_last, inv, rho);
+    auto it = T.tw.find(key);
     if (it != T.tw.end()) { *out = it->second; return VI_OK; }
-    std::vector<uint64_t> h((size_t)n);
-    uint64_t wn = vgl::hpow(7, (vgl::P - 1) / (uint64_t)n), cur = 1;
-    for (int64_t e = 0; e < n; ++e) { h[(size_t)e] = cur; cur = vgl::hmul(cur, wn); }
     uint64_t* d = nullptr;
-    int rc_up = upload_table(h, &d);
+    int rc_up = upload_table(small_last ? stage_twiddles<true>(logl, inv, rho) : stage_twiddles<false>(logl, inv, rho), &d);
     if (rc_up) return rc_up;
-    T.tw[n] = d;
+    T.tw[key] = d;
     *out = d;
     return VI_OK;
 }
@@ -769,7 +782,7 @@ int launch_pass_l(int logL, const PassArgs& a, int64_t items, cudaStream_t st, i
 
 int launch_pass(int logL, bool inv, int mode, PassArgs& a, int64_t items, cudaStream_t st, int tag) {
     a.tiles_per_item = (a.ncols + (1 << a.logC) - 1) >> a.logC;
-    int rc = get_tw(int64_t(1) << logL, &a.twL);
+    int rc = get_tw(logL, false, inv, 0, &a.tw);
     if (rc) return rc;
     if (inv) return mode ? launch_pass_l<true, 1>(logL, a, items, st, tag) : launch_pass_l<true, 0>(logL, a, items, st, tag);
     return mode ? launch_pass_l<false, 1>(logL, a, items, st, tag) : launch_pass_l<false, 0>(logL, a, items, st, tag);
@@ -887,7 +900,7 @@ extern "C" int vi_ntt_batched(uint64_t* rows, int64_t m, int64_t n, int inverse,
             a.in = rows + r * n; a.out = s1;
             a.logC = pick_logC(log1, n2);
             a.ncols = n2;
-            a.in_item = 0; a.in_idx = (uint32_t)n2; a.in_col = 1;
+            a.in_item = 0; a.in_idx = (uint32_t)n2;
             a.out_item = 0; a.out_k = (uint32_t)n2; a.out_col = 1;
             a.fs = flo; a.fs_hi = fhi; a.scale = 1; a.out_via_smem = 0; a.src_kind = SRC_PLAIN;
             rc = launch_pass(log1, inv, 0, a, 1, st, vi::PROF_NTT_PASS);
@@ -896,7 +909,7 @@ extern "C" int vi_ntt_batched(uint64_t* rows, int64_t m, int64_t n, int inverse,
             b.in = s1; b.out = s2;
             b.logC = pick_logC(loga, nb);
             b.ncols = nb;
-            b.in_item = n2; b.in_idx = (uint32_t)nb; b.in_col = 1;
+            b.in_item = n2; b.in_idx = (uint32_t)nb;
             b.out_item = n2; b.out_k = (uint32_t)nb; b.out_col = 1;
             b.fs = fs2; b.scale = 1; b.out_via_smem = 0; b.src_kind = SRC_PLAIN;
             rc = launch_pass(loga, inv, 0, b, n1, st, vi::PROF_NTT_PASS);
@@ -905,7 +918,7 @@ extern "C" int vi_ntt_batched(uint64_t* rows, int64_t m, int64_t n, int inverse,
             c.in = s2; c.out = rows + r * n;
             c.logC = pick_logC(logb, na);
             c.ncols = na;
-            c.in_item = n2; c.in_idx = 1; c.in_col = (uint32_t)nb;
+            c.in_item = n2;
             c.out_item = 1; c.out_k = (uint32_t)(n1 * na); c.out_col = (uint32_t)n1;
             c.fs = nullptr; c.scale = scale; c.out_via_smem = 0; c.src_kind = SRC_PLAIN;
             rc = launch_pass(logb, inv, 1, c, n1, st, vi::PROF_NTT_PASS);
@@ -918,7 +931,7 @@ extern "C" int vi_ntt_batched(uint64_t* rows, int64_t m, int64_t n, int inverse,
         a.in = rows; a.out = rows;
         a.logC = pick_logC(logn, m);
         a.ncols = m;
-        a.in_item = 0; a.in_idx = 1; a.in_col = (uint32_t)n;
+        a.in_item = 0;
         a.out_item = 0; a.out_k = 1; a.out_col = (uint32_t)n;
         a.fs = nullptr; a.scale = scale; a.out_via_smem = 1; a.src_kind = SRC_PLAIN;
         return launch_pass(logn, inv, 1, a, 1, st, vi::PROF_NTT_PASS);
@@ -937,7 +950,7 @@ extern "C" int vi_ntt_batched(uint64_t* rows, int64_t m, int64_t n, int inverse,
         a.in = rows + r0 * n; a.out = (uint64_t*)scratch;
         a.logC = pick_logC(log1, n2);
         a.ncols = n2;
-        a.in_item = n; a.in_idx = (uint32_t)n2; a.in_col = 1;
+        a.in_item = n; a.in_idx = (uint32_t)n2;
         a.out_item = n; a.out_k = (uint32_t)n2; a.out_col = 1;
         a.fs = fsn; a.scale = 1; a.out_via_smem = 0; a.src_kind = SRC_PLAIN;
         rc = launch_pass(log1, inv, 0, a, cnt, st, vi::PROF_NTT_PASS);
@@ -946,7 +959,7 @@ extern "C" int vi_ntt_batched(uint64_t* rows, int64_t m, int64_t n, int inverse,
         b.in = (const uint64_t*)scratch; b.out = rows + r0 * n;
         b.logC = pick_logC(log2, n1);
         b.ncols = n1;
-        b.in_item = n; b.in_idx = 1; b.in_col = (uint32_t)n2;
+        b.in_item = n;
         b.out_item = n; b.out_k = (uint32_t)n1; b.out_col = 1;
         b.fs = nullptr; b.scale = scale; b.out_via_smem = 0; b.src_kind = SRC_PLAIN;
         rc = launch_pass(log2, inv, 1, b, cnt, st, vi::PROF_NTT_PASS);
@@ -990,7 +1003,7 @@ extern "C" int vi_ntt_forward_padded(const uint64_t* src, int64_t m, int64_t k_i
         a.in = src + r0 * k_in; a.out = (uint64_t*)scratch;
         a.logC = pick_logC(log1, n2);
         a.ncols = n2;
-        a.in_item = k_in; a.in_idx = (uint32_t)n2; a.in_col = 1;
+        a.in_item = k_in; a.in_idx = (uint32_t)n2;
         a.out_item = n; a.out_k = (uint32_t)n2; a.out_col = 1;
         a.fs = fsn; a.scale = 1; a.out_via_smem = 0;
         a.src_kind = SRC_MSG; a.ell = k_in; a.pad_mode = 0;
@@ -1000,7 +1013,7 @@ extern "C" int vi_ntt_forward_padded(const uint64_t* src, int64_t m, int64_t k_i
         b.in = (const uint64_t*)scratch; b.out = dst + r0 * n;
         b.logC = pick_logC(log2, n1);
         b.ncols = n1;
-        b.in_item = n; b.in_idx = 1; b.in_col = (uint32_t)n2;
+        b.in_item = n;
         b.out_item = n; b.out_k = (uint32_t)n1; b.out_col = 1;
         b.fs = nullptr; b.scale = 1; b.out_via_smem = 0; b.src_kind = SRC_PLAIN;
         rc = launch_pass(log2, false, 1, b, cnt, st, vi::PROF_NTT_PASS);
@@ -1053,11 +1066,10 @@ static int encode_impl(const uint64_t* msg, const KqSrc* kq, int64_t m, int64_t 
     const uint64_t *fs_inv, *fs_fwd = nullptr, *twist = nullptr;
     int rc = get_fs(k, n2, true, &fs_inv);        // inverse step 1: columns j2 (n2 of them), index k1
     if (rc) return rc;
-    const uint64_t *cscale = nullptr, *twRL = nullptr, *fsN = nullptr;
+    const uint64_t *cscale = nullptr, *fsN = nullptr;
     const bool shift_form = codes && mid_shift_form(log2, rho);
     if (shift_form) {
         rc = get_cscale(k, &cscale); if (rc) return rc;
-        rc = get_tw(rho * n2, &twRL); if (rc) return rc;
         rc = get_fs(n, n1, false, &fsN); if (rc) return rc;                  // w_N^(l2*(rho*m1 + t))
     } else if (codes) {
         rc = get_fs(k, n1, false, &fs_fwd); if (rc) return rc;               // forward step 1: columns l2 (n1), index m1
@@ -1072,7 +1084,7 @@ static int encode_impl(const uint64_t* msg, const KqSrc* kq, int64_t m, int64_t 
         a.in = kq ? nullptr : msg + r0 * ell; a.out = s1;
         a.logC = pick_logC(log1, n2);
         a.ncols = n2;
-        a.in_item = ell; a.in_idx = (uint32_t)n2; a.in_col = 1;
+        a.in_item = ell; a.in_idx = (uint32_t)n2;
         a.out_item = k; a.out_k = (uint32_t)n2; a.out_col = 1;
         a.fs = fs_inv; a.scale = 1; a.out_via_smem = 0;
         a.src_kind = kq ? SRC_KQ : SRC_MSG; a.ell = ell;
@@ -1094,8 +1106,10 @@ static int encode_impl(const uint64_t* msg, const KqSrc* kq, int64_t m, int64_t 
         mid.n1 = n1; mid.tiles_per_item = (n1 + (1 << mid.logC) - 1) >> mid.logC;
         VI_REQUIRE(fixed_logC(log2) < 0 || n1 % (int64_t(1) << mid.logC) == 0, "encode: internal tile shape");
         mid.rho = (int)rho; mid.K = k; mid.fsK = fs_fwd; mid.twist = twist; mid.k_inv = inv_pow2(logk);
-        mid.cscale = cscale; mid.twRL = twRL; mid.fsN = fsN;
-        rc = get_tw(n2, &mid.twL);
+        mid.cscale = cscale; mid.fsN = fsN;
+        rc = get_tw(log2, false, true, 0, &mid.tw_inv);
+        if (rc) return rc;
+        rc = get_tw(log2, true, false, shift_form ? (int)rho : 0, &mid.tw_fwd);
         if (rc) return rc;
         rc = launch_mid(log2, mid, cnt, st);
         if (rc) return rc;
@@ -1105,7 +1119,7 @@ static int encode_impl(const uint64_t* msg, const KqSrc* kq, int64_t m, int64_t 
         b.in = s2; b.out = codes + r0 * n;
         b.ncols = rho * n2;
         b.logC = pick_logC(log1, b.ncols);
-        b.in_item = n; b.in_idx = 1; b.in_col = (uint32_t)n1;
+        b.in_item = n;
         b.out_item = n; b.out_k = (uint32_t)(rho * n2); b.out_col = 1;
         b.fs = nullptr; b.scale = 1; b.out_via_smem = 0; b.src_kind = SRC_PLAIN;
         rc = launch_pass(log1, false, 1, b, cnt, st, vi::PROF_ENC_PASS3);
