@@ -12,7 +12,8 @@
  *    process and never traps the device.
  *  - The only memory the library owns are immutable per-device twiddle tables,
  *    allocated (cudaMalloc + synchronous upload) the first time a transform
- *    length is used on a device.
+ *    length is used on a device, and up to 32 small result buffers (4 KB of mapped
+ *    host memory each) per device that sumcheck proofs take turns with.
  *
  * Each declaration cites the reference interface it replaces (paths relative to
  * the reference project root).  A ctypes binding of these symbols is what the
@@ -57,7 +58,7 @@ int vi_ntt_batched(uint64_t* rows, int64_t m, int64_t n, int inverse,
 /* The library owns only immutable per-device tables (twiddles, four-step factors, coset
  * scalings), built on the first use of a length and kept for the life of the process, as the
  * reference keeps its twiddle contexts (prover/cuda_primitives.py:319-331).  vi_release_tables
- * frees them all; call it with no library kernel in flight. */
+ * frees them all (and the idle sumcheck result buffers); call it with no library kernel in flight. */
 int vi_release_tables(void);
 
 /* ---- Reed-Solomon row encode ---------------------------------------------------
@@ -247,6 +248,28 @@ int vi_sumcheck_round(uint64_t* tables, int64_t stride, int n_tables, int64_t si
  * coins: HOST array of n_rounds canonical challenges; n_rounds <= 64, 1 <= deg <= 7.  Row 0 must be
  * complete.  One launch of one CTA; lets the caller copy finished round polynomials in one transfer. */
 int vi_sumcheck_complete(uint64_t* samples, int n_rounds, int deg, const uint64_t* coins, void* stream);
+
+/* Whole proofs from tables that stay where and as they are (HOST array `tables` of n_tables device pointers, `size`
+ * entries each): replaces prove_terms_gpu with its per-round copies and folds (layergkr/gpu.py:350-410).
+ *   vi_sumcheck_prove   challenges known up front (HOST coins[n_rounds], size = 2^n_rounds).  Waits for the stream and
+ *                       writes the complete g(0..deg) of round i to samples_host[8*i ..] (HOST).  Round 0's
+ *                       g(0) + g(1) is the claim.
+ *   vi_sumcheck_open / _step / _close   one round per call: the first step gives round 0 (its r is ignored), every later
+ *                       one folds with r, the challenge of the round before, and gives the next round's g(0..deg);
+ *                       log2(size) steps in all.  A session is used by one thread at a time.
+ * work: device memory of vi_sumcheck_prove_work_bytes / vi_sumcheck_session_work_bytes bytes, 8-byte aligned, that
+ * stays with the call or the session. */
+int64_t vi_sumcheck_prove_work_bytes(int n_tables, int64_t size);
+int vi_sumcheck_prove(const uint64_t* const* tables, int n_tables, int64_t size,
+                      int n_terms, const uint64_t* coefs, const int32_t* nfac, const int32_t* fac,
+                      const uint64_t* coins, int n_rounds, void* work, int64_t work_bytes,
+                      uint64_t* samples_host, void* stream);
+int64_t vi_sumcheck_session_work_bytes(int n_tables, int64_t size);
+int vi_sumcheck_open(const uint64_t* const* tables, int n_tables, int64_t size,
+                     int n_terms, const uint64_t* coefs, const int32_t* nfac, const int32_t* fac,
+                     void* work, int64_t work_bytes, void* stream, void** session);
+int vi_sumcheck_step(void* session, uint64_t r, uint64_t* samples_host);
+int vi_sumcheck_close(void* session);
 
 /* ---- remaining exports of the reference module (not on the hot path) -------------
  * poly_eval (prover/kernels/gl_extras.cuh:93-108), gl_matmul / gl_matvec

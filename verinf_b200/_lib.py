@@ -55,6 +55,12 @@ SIGNATURES = {
     "vi_sumcheck_run": (_int, [_p, _i64, _int, _i64, _int, _p, _p, _p, _p, _int, _p, _p, _p]),
     "vi_sumcheck_round": (_int, [_p, _i64, _int, _i64, _int, _p, _p, _p, _int, _u64, _p, _p, _p]),
     "vi_sumcheck_complete": (_int, [_p, _int, _int, _p, _p]),
+    "vi_sumcheck_prove_work_bytes": (_i64, [_int, _i64]),
+    "vi_sumcheck_prove": (_int, [_p, _int, _i64, _int, _p, _p, _p, _p, _int, _p, _i64, _p, _p]),
+    "vi_sumcheck_session_work_bytes": (_i64, [_int, _i64]),
+    "vi_sumcheck_open": (_int, [_p, _int, _i64, _int, _p, _p, _p, _p, _i64, _p, _p]),
+    "vi_sumcheck_step": (_int, [_p, _u64, _p]),
+    "vi_sumcheck_close": (_int, [_p]),
     "vi_poly_eval": (_int, [_p, _i64, _i64, _p, _i64, _p, _p]),
     "vi_gl_matmul": (_int, [_p, _p, _p, _i64, _i64, _i64, _p]),
     "vi_gl_matmul_tc_scratch_bytes": (_i64, [_i64, _i64, _i64]),

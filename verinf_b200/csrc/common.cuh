@@ -17,6 +17,7 @@ namespace vi {
 
 int fail(int code, const char* fmt, ...);   // records the message, returns code
 int check_launch(const char* what);          // cudaGetLastError -> status
+void release_sumcheck_slots();               // frees the idle result buffers of sumcheck_prove.cu
 
 // Optional per-kernel timing with CUDA events on the launching stream (off by default).
 enum ProfTag { PROF_ENC_PASS1 = 0, PROF_ENC_MID, PROF_ENC_PASS3, PROF_NTT_PASS, PROF_HASH, PROF_MERKLE,

@@ -852,6 +852,7 @@ extern "C" int vi_release_tables(void) {
         for (auto& t : kv.second.split) { cudaFree(t.second.first); cudaFree(t.second.second); }
     }
     g_tables.clear();
+    vi::release_sumcheck_slots();
     VI_CUDA(cudaSetDevice(cur));
     return VI_OK;
 }

@@ -5,9 +5,10 @@ and return values): `encode_batch_ntt`, `hash_and_tree`, `prove_terms_gpu` on th
 `fold_t`, layergkr/gpu.py:92-126, 256-347), so the module can stand in for layergkr.gpu.
 
 `prove_terms_gpu` keeps the reference's per-round `coin` callback, but each round is one
-fused fold+evaluate launch and one small D2H copy of the deg+1 samples, instead of ~10
-elementwise launches and a host sync per sample point.
+fused fold+evaluate launch that hands its sums to the host, instead of ~10 elementwise
+launches and a host sync per sample point, and the caller's tables are read where they are.
 """
+import ctypes as C
 from typing import Callable, List, Optional, Sequence
 
 import numpy as np
@@ -241,12 +242,63 @@ class SumcheckProblem:
 _MAX_TABLES, _MAX_TERMS = 8, 8          # per launch of the sumcheck kernels (csrc/sumcheck.cu)
 
 
+class _Plan:
+    """Up to _MAX_TABLES tables (1-D uint64 CUDA tensors, read in place) and _MAX_TERMS terms as the C ABI takes them."""
+
+    def __init__(self, tables: Sequence[torch.Tensor], terms: Sequence):
+        self.tables, self.dev, self.size = tables, tables[0].device, tables[0].numel()
+        if any(t.numel() != self.size or t.device != self.dev for t in tables):
+            raise RuntimeError("sumcheck: tables of different sizes or devices")
+        self.deg = max(len(f) for _, f in terms)
+        n = len(terms)
+        if self.deg > _MAX_FAC:
+            raise RuntimeError(f"sumcheck: at most {_MAX_FAC} factors per term")
+        fac = [0] * (n * _MAX_FAC)
+        for t, (_, f) in enumerate(terms):
+            fac[t * _MAX_FAC:t * _MAX_FAC + len(f)] = f
+        self._args = ((C.c_void_p * len(tables))(*[t.data_ptr() for t in tables]), len(tables), self.size, n,
+                      (C.c_uint64 * n)(*[c for c, _ in terms]), (C.c_int32 * n)(*[len(f) for _, f in terms]),
+                      (C.c_int32 * len(fac))(*fac))
+        self._session = None
+
+    def _work(self, nbytes):
+        return torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
+
+    def run(self, coins: Sequence[int]) -> List[List[int]]:
+        """g(0..deg) of every round, all challenges known (canonical): one wait for the device."""
+        n = len(coins)
+        out = (C.c_uint64 * (8 * n))()
+        nb = LIB.vi_sumcheck_prove_work_bytes(len(self.tables), self.size)
+        with torch.cuda.device(self.dev):
+            work = self._work(nb)
+            check(LIB.vi_sumcheck_prove(*self._args, (C.c_uint64 * n)(*coins), n, work.data_ptr(), nb, out, stream_ptr()))
+        d = self.deg + 1
+        return [out[8 * i:8 * i + d] for i in range(n)]
+
+    def round(self, r: Optional[int]) -> List[int]:
+        """Round 0 with r None, then one round per challenge; the last challenge folds nothing that is read."""
+        if self._session is None:
+            self._out = (C.c_uint64 * 8)()
+            h = C.c_void_p()
+            nb = LIB.vi_sumcheck_session_work_bytes(len(self.tables), self.size)
+            with torch.cuda.device(self.dev):
+                self._buf = self._work(nb)
+                check(LIB.vi_sumcheck_open(*self._args, self._buf.data_ptr(), nb, stream_ptr(), C.byref(h)))
+            self._session = h
+        check(LIB.vi_sumcheck_step(self._session, r or 0, self._out))
+        return self._out[:self.deg + 1]
+
+    def close(self):
+        if self._session is not None:
+            LIB.vi_sumcheck_close(self._session)
+            self._session = None
+
+
 class TermGroups:
     """A sum of products with more tables or terms than one kernel launch takes (a layer's gate batch,
     layergkr/relations.py:103-124, has hundreds): the sum is linear in its terms, so the terms are split
-    into groups that fit, every group is its own SumcheckProblem folded with the same challenges, and the
-    round samples are added.  A group of lower degree is extended to the common number of samples by
-    evaluating its round polynomial at the further nodes.  Same interface as SumcheckProblem."""
+    into groups that fit, every group is folded with the same challenges, and the round samples are added.  A group of
+    lower degree is extended to the common number of samples by evaluating its round polynomial at the further nodes."""
 
     def __init__(self, rows: Sequence[torch.Tensor], plan: Sequence):
         self.deg = max(len(idx) for _, idx in plan)
@@ -258,13 +310,12 @@ class TermGroups:
             cur.append((c, idx))
             used |= set(idx)
         groups.append(cur)
-        self.problems = []
+        self.plans = []
         for g in groups:
             need = sorted({i for _, idx in g for i in idx})
             at = {t: j for j, t in enumerate(need)}
-            tables = torch.stack([rows[t].view(torch.int64) for t in need]).view(torch.uint64).contiguous()
-            self.problems.append(SumcheckProblem(tables, [(c, [at[i] for i in idx]) for c, idx in g]))
-        self.size = self.problems[0].size
+            self.plans.append(_Plan([rows[t] for t in need], [(c, [at[i] for i in idx]) for c, idx in g]))
+        self.size = self.plans[0].size
 
     def _add(self, per_group: Sequence[List[int]]) -> List[int]:
         n = self.deg + 1
@@ -274,18 +325,16 @@ class TermGroups:
             out = [(a + b) % P for a, b in zip(out, ys)]
         return out
 
-    def claim(self) -> int:
-        return sum(p.claim() for p in self.problems) % P
-
-    def round(self, r: Optional[int]) -> Optional[List[int]]:
-        res = [p.round(r) for p in self.problems]
-        self.size = self.problems[0].size
-        return None if res[0] is None else self._add(res)
+    def round(self, r: Optional[int]) -> List[int]:
+        return self._add([p.round(r) for p in self.plans])
 
     def run(self, coins: Sequence[int]) -> List[List[int]]:
-        per = [p.run(coins) for p in self.problems]
-        self.size = 1
+        per = [p.run(coins) for p in self.plans]
         return [self._add([g[i] for g in per]) for i in range(len(coins))]
+
+    def close(self):
+        for p in self.plans:
+            p.close()
 
 
 def samples_to_host(buf: torch.Tensor, deg: int) -> List[List[int]]:
@@ -358,45 +407,65 @@ def prove_terms_gpu(terms, coin: Callable[[int], int], field_p: int = P, mask=No
     rows = []
     for f in uniq:
         if isinstance(f, torch.Tensor):
-            rows.append(f.to(device="cuda").reshape(-1))
+            if not f.is_cuda:
+                f = f.to(device="cuda")
+            rows.append(f.reshape(-1) if f.dim() != 1 else f)
+            if not rows[-1].is_contiguous():
+                rows[-1] = rows[-1].contiguous()
         else:
             rows.append(torch.tensor([int(x) % P for x in f], dtype=torch.uint64, device="cuda"))
-    if len(rows) > _MAX_TABLES or len(plan) > _MAX_TERMS:
-        prob = TermGroups(rows, plan)
-    else:
-        tables = torch.stack([r.view(torch.int64) for r in rows]).view(torch.uint64).contiguous()
-        prob = SumcheckProblem(tables, plan)
-    n_rounds = prob.size.bit_length() - 1
-    deg = prob.deg
+        if rows[-1].dtype != torch.uint64:
+            raise RuntimeError("sumcheck: tables must be uint64")
+    if len({r.numel() for r in rows}) != 1:
+        raise RuntimeError("sumcheck: tables of different sizes")
     mu = mu0 % P
+    n_rounds = rows[0].numel().bit_length() - 1
+    if n_rounds == 0:              # single entries: the claim is the sum of the terms, and there is no round
+        prob = SumcheckProblem(torch.stack([r.view(torch.int64) for r in rows]).view(torch.uint64), [(1, [0])])
+        vals = prob.finals()
+        claim = mu
+        for c, idx in plan:
+            for i in idx:
+                c = c * vals[i] % P
+            claim += c
+        return claim % P, [], [], mu
+    prob = TermGroups(rows, plan) if len(rows) > _MAX_TABLES or len(plan) > _MAX_TERMS else _Plan(rows, plan)
+    deg = prob.deg
     round_polys, challenges = [], []
+
+    def masked(samples):
+        """A round's samples with the mask polynomial added, and the mask's coefficients."""
+        h = mask(deg, mu)
+        return [(x, (y + _poly_eval(h, x, P)) % P) for x, y in samples], h
+
     if coins is None and predraw:
         coins = [coin(rnd) for rnd in range(n_rounds)]
-    if coins is not None and n_rounds > 0:
+    if coins is not None:
         challenges = [int(c) % P for c in coins]
+        assert len(challenges) == n_rounds
         all_ys = prob.run(challenges)
         claim = (all_ys[0][0] + all_ys[0][1] + mu) % P       # the sum over the hypercube is g_0(0) + g_0(1)
         for ys, r in zip(all_ys, challenges):
             samples = list(enumerate(ys))
             if mask is not None:
-                h = mask(deg, mu)
-                samples = [(x, (y + _poly_eval(h, x, P)) % P) for x, y in samples]
+                samples, h = masked(samples)
                 mu = _poly_eval(h, r, P)
             round_polys.append(samples)
         return claim, round_polys, challenges, mu
-    claim = (prob.claim() + mu) % P
     r = None
-    for rnd in range(n_rounds):
-        ys = prob.round(r)
-        samples = list(enumerate(ys))
-        if mask is not None:
-            h = mask(deg, mu)
-            samples = [(x, (y + _poly_eval(h, x, P)) % P) for x, y in samples]
-        round_polys.append(samples)
-        r = coin(rnd) % P
-        challenges.append(r)
-        if mask is not None:
-            mu = _poly_eval(h, r, P)
-    if n_rounds:
-        prob.round(r)          # last fold: tables collapse to their evaluation at the challenge point
+    try:
+        for rnd in range(n_rounds):
+            ys = prob.round(r)
+            if rnd == 0:
+                claim = (ys[0] + ys[1] + mu) % P
+            samples = list(enumerate(ys))
+            if mask is not None:
+                samples, h = masked(samples)
+            round_polys.append(samples)
+            r = coin(rnd) % P
+            challenges.append(r)
+            if mask is not None:
+                mu = _poly_eval(h, r, P)
+    finally:
+        prob.close()
     return claim, round_polys, challenges, mu
