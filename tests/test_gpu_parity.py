@@ -243,6 +243,20 @@ def test_encode_vs_oracle(cp, ell, k, n, m, pad):
             assert torch.equal(ext.view(torch.int64), codes.view(torch.int64))
 
 
+@pytest.mark.parametrize("k,n,m", [(2, 16, 1), (64, 64, 3), (256, 512, 5), (256, 4096, 7), (512, 2048, 64), (1024, 2048, 1),
+                                   (1024, 4096, 70), (1024, 8192, 2), (2048, 8192, 9), (4096, 16384, 2), (8192, 65536, 1),
+                                   (16384, 65536, 1), (16384, 32768, 37)])
+def test_encode_few_tiles(cp, k, n, m):
+    """too few tiles for the GPU: cosets of a tile dealt out to CTAs, tiles cut down to 16 columns; blow-ups 1 to 16"""
+    rng = np.random.default_rng(k + n + m)
+    msg = rnd_field(rng, (m, k))
+    want_p, want_c = oracle.encode_rows(msg, n)
+    polys, codes = cp.encode_rows(dev(msg), k, n)
+    assert np.array_equal(host(polys), want_p) and np.array_equal(host(codes), want_c)
+    _, c2 = cp.encode_rows(dev(msg), k, n, need_polys=False)
+    assert np.array_equal(host(c2), want_c)
+
+
 @pytest.mark.parametrize("ell,k,n,m", [((1 << 21) - 5, 1 << 21, 1 << 22, 2), (1 << 23, 1 << 23, 1 << 24, 1)])
 def test_encode_long_rows(cp, ell, k, n, m):
     """K above 2^20: tile DFT lengths 2048 and 4096 (4 and 2 columns per tile)"""
@@ -308,7 +322,8 @@ def test_hash_golden(cp, golden):
 
 
 @pytest.mark.parametrize("m,n", [(1, 1), (5, 33), (128, 100), (129, 100), (255, 7), (256, 64), (257, 64),
-                                 (1000, 300), (4096, 64), (4224, 40), (16385, 9)])
+                                 (1000, 300), (4096, 64), (4224, 40), (16385, 9), (0, 5), (7, 200), (8, 37888), (9, 37889),
+                                 (63, 4096), (64, 4096), (127, 130), (384, 2000), (385, 2000), (500, 70000), (1025, 130)])
 def test_hash_columns_vs_oracle(cp, m, n):
     rng = np.random.default_rng(m * 31 + n)
     a = rnd_field(rng, (m, n))
@@ -335,7 +350,7 @@ def test_merkle_column_accumulator(cp, total, pieces):
         cp.MerkleColumnAccumulator(n, 128)
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 5, 8, 1000, 1024, 4097])
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 8, 31, 64, 65, 511, 512, 513, 1000, 1024, 1025, 4097, 65537, 262144, 262147])
 def test_merkle_vs_oracle(cp, n):
     rng = np.random.default_rng(n)
     leaves = rng.integers(0, 256, size=(n, 32), dtype=np.uint8)
@@ -553,7 +568,116 @@ def test_sumcheck_many_tables_and_terms_vs_oracle(logn, nt, nterms, predraw):
     assert [[y for _, y in rp] for rp in got[1]] == [[int(v) for v in row[:5]] for row in samples]
 
 
+_SHAPES = [[(1, [0, 1])], [(1, [0, 1, 2])], [(1, [0])], [(1, [0, 1, 2, 3])], [(1, [0, 1, 2]), (P - 1, [0, 3])],
+           [(7, [0, 0, 1]), (P - 1, [2]), (5, [1, 3, 3, 3])]]
+
+
+@pytest.mark.parametrize("logn", [1, 2, 3, 8, 9, 10, 11, 12, 13, 17])
+@pytest.mark.parametrize("terms", range(len(_SHAPES)))
+def test_whole_proofs_vs_oracle(logn, terms):
+    """Proofs from the caller's tables, challenges known and one at a time: product terms and general ones, sizes around
+    the one-block and the host rounds, entries 0 and p - 1 in the first pair of every table; tables left as they are."""
+    from verinf_b200 import layergkr_gpu as lg
+    shape = _SHAPES[terms]
+    nt = 1 + max(i for _, f in shape for i in f)
+    rng = np.random.default_rng(31 * logn + terms)
+    tabs = rnd_field(rng, (nt, 1 << logn))
+    tabs[:, 0], tabs[:, -1] = 0, P - 1
+    coins = [int(c) for c in rnd_field(rng, logn)]
+    coins[0] = P - 1
+    claim, samples, _ = oracle.sumcheck(tabs, shape, coins)
+    deg = max(len(f) for _, f in shape)
+    want = [[int(v) for v in row[:deg + 1]] for row in samples]
+    dts = [dev(t) for t in tabs]
+    plan = [(c, [dts[i] for i in f]) for c, f in shape]
+    for kw in (dict(), dict(coins=coins), dict()):          # the result buffers of one proof serve the next
+        got = lg.prove_terms_gpu(plan, lambda i: coins[i], **kw)
+        assert got[0] == claim and [[y for _, y in rp] for rp in got[1]] == want
+    assert all(np.array_equal(host(d), t) for d, t in zip(dts, tabs))
+
+
+def test_whole_proofs_take_tables_as_before():
+    """words of another 8-byte type, strided and 2-D tables, and a proof per thread and stream at once"""
+    import threading
+    from verinf_b200 import layergkr_gpu as lg
+    rng = np.random.default_rng(77)
+    tabs = rnd_field(rng, (2, 4096))
+    coins = [int(c) for c in rnd_field(rng, 12)]
+    claim, samples, _ = oracle.sumcheck(tabs, [(1, [0, 1])], coins)
+    want = [[int(v) for v in row[:3]] for row in samples]
+    a, b = dev(tabs[0]), dev(tabs[1])
+    wide = torch.zeros((4096, 2), dtype=torch.int64, device="cuda")
+    wide[:, 0] = a.view(torch.int64)
+    for f in (a.view(torch.int64), a.view(torch.float64), a.reshape(64, 64), wide[:, 0]):
+        got = lg.prove_terms_gpu([(1, [f, b])], lambda i: coins[i])
+        assert got[0] == claim and [[y for _, y in rp] for rp in got[1]] == want
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for rep in range(5):
+                kw = dict(coins=coins) if (i + rep) % 2 else {}
+                got = lg.prove_terms_gpu([(1, [a, b])], lambda j: coins[j], **kw)
+                if got[0] != claim or [[y for _, y in rp] for rp in got[1]] != want:
+                    bad.append((i, rep))
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    assert not bad
+
+
 # ---------------------------------------------------------------- misc ops ---
+@pytest.mark.parametrize("m,n", [(3, 255), (3, 256), (3, 511), (3, 512), (3, 513), (2, 1025), (1, 2048), (3, 2303), (2, 4097),
+                                 (4736, 520), (4737, 520), (1, 1)])
+def test_matvec_row_shares(cp, m, n):
+    """one to eight warps per row; the batched loads and the remainder behind them"""
+    rng = np.random.default_rng(m + n)
+    M, v = rnd_field(rng, (m, n)), rnd_field(rng, n)
+    M[0] = P - 1
+    v[:] = np.where(np.arange(n) % 2 == 0, np.uint64(P - 1), v)
+    want = oracle.gl_matmul(M, v.reshape(-1, 1))
+    assert np.array_equal(host(cp.gl_matvec(dev(M), dev(v))), want[:, 0])
+    off = torch.zeros(m * n + 1, dtype=torch.int64, device="cuda").view(torch.uint64)        # rows off 16-byte boundaries
+    off.view(torch.int64)[1:] = dev(M).view(torch.int64).reshape(-1)
+    assert np.array_equal(host(cp.gl_matvec(off[1:].view(m, n), dev(v))), want[:, 0])
+    assert np.array_equal(host(cp.gl_matmul(dev(M), dev(v.reshape(-1, 1)))), want)
+
+
+@pytest.mark.parametrize("k", [1, 7, 31, 63, 64, 65, 127, 255, 256, 300, 1000])
+@pytest.mark.parametrize("n", [2, 31, 33, 100, 5000, 38000])
+def test_thin_product_clusters(cp, k, n):
+    """one to eight CTAs per 32 columns, rows that do not fill a batch, a last column block that is not full"""
+    rng = np.random.default_rng(k * 7 + n)
+    B = rnd_field(rng, (k, n))
+    B[0] = P - 1
+    for m in (1, 2, 3, 4):
+        A = rnd_field(rng, (m, k))
+        A[:, 0] = P - 1
+        assert np.array_equal(host(cp.gl_matmul(dev(A), dev(B))), oracle.gl_matmul(A, B))
+
+
+def test_product_colsum_with_less_scratch(cp):
+    """the row splits follow the scratch that is there, down to what earlier callers were asked for"""
+    from verinf_b200._lib import LIB, check, ptr, stream_ptr
+    rng = np.random.default_rng(4)
+    T, n = 1003, 5000
+    EA, EB, w = rnd_field(rng, (T, n)), rnd_field(rng, (T, n)), rnd_field(rng, T)
+    a, b, wd = dev(EA), dev(EB), dev(w)
+    full, least = LIB.vi_product_colsum_scratch_bytes(T, n), 30 * n * 8       # 148 * 4 CTAs of 256 columns
+    outs = []
+    for nb in (full, max(full - 8, least), least + 16, least):
+        sc = torch.empty(nb, dtype=torch.uint8, device="cuda")
+        out = torch.zeros(n, dtype=torch.uint64, device="cuda")
+        check(LIB.vi_product_colsum(ptr(a), ptr(b), n, None, None, ptr(wd), T, ptr(out), 0, ptr(sc), nb, stream_ptr()))
+        outs.append(host(out))
+    assert all(np.array_equal(o, outs[0]) for o in outs)
+    at = [0, 255, 256, n - 1]
+    ref = [sum(int(x) * int(y) * int(z) for x, y, z in zip(w, EA[:, j], EB[:, j])) % P for j in at]
+    assert [int(outs[0][j]) for j in at] == ref
+    assert LIB.vi_product_colsum(ptr(a), ptr(b), n, None, None, ptr(wd), T, ptr(out), 0, ptr(sc), least - 8, stream_ptr()) != 0
+
+
 def test_linear_algebra(cp):
     rng = np.random.default_rng(5)
     A, B = rnd_field(rng, (37, 65)), rnd_field(rng, (65, 41))
@@ -750,6 +874,17 @@ def test_matmul_tcgen05_vs_oracle(cp, m, k, n):
     rng = np.random.default_rng(m * 11 + k + n)
     A, B = rnd_field(rng, (m, k)), rnd_field(rng, (k, n))
     assert np.array_equal(_matmul_umma(A, B), oracle.gl_matmul(A, B))
+
+
+@pytest.mark.parametrize("m,k,n", [(2179, 33, 290), (130, 4100, 2530), (129, 8224, 2400), (2048, 31, 321)])
+def test_matmul_tcgen05_more_tiles_than_sms(cp, m, k, n):
+    """more tiles than SMs, with one or more 4096-term chunks each, row tiles in a full and a ragged group of 16, k next to
+    a multiple of 32; the oracle on a choice of rows"""
+    rng = np.random.default_rng(m + k + n)
+    A, B = rnd_field(rng, (m, k)), rnd_field(rng, (k, n))
+    got = _matmul_umma(A, B)
+    at = np.unique(np.concatenate([[0, 1, m - 1, m // 2], rng.integers(0, m, size=6)]))
+    assert np.array_equal(got[at], oracle.gl_matmul(A[at], B))
 
 
 def test_matmul_tcgen05_extreme_operands_and_dispatch(cp):

@@ -407,15 +407,12 @@ def prove_terms_gpu(terms, coin: Callable[[int], int], field_p: int = P, mask=No
     rows = []
     for f in uniq:
         if isinstance(f, torch.Tensor):
-            if not f.is_cuda:
-                f = f.to(device="cuda")
-            rows.append(f.reshape(-1) if f.dim() != 1 else f)
-            if not rows[-1].is_contiguous():
-                rows[-1] = rows[-1].contiguous()
+            f = f.to(device="cuda").reshape(-1)
+            if f.dtype != torch.uint64:       # the words of another type, eight bytes each
+                f = f.view(torch.int64).view(torch.uint64)
+            rows.append(f.contiguous())
         else:
             rows.append(torch.tensor([int(x) % P for x in f], dtype=torch.uint64, device="cuda"))
-        if rows[-1].dtype != torch.uint64:
-            raise RuntimeError("sumcheck: tables must be uint64")
     if len({r.numel() for r in rows}) != 1:
         raise RuntimeError("sumcheck: tables of different sizes")
     mu = mu0 % P
