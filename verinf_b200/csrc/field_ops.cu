@@ -12,10 +12,13 @@
 // prover/kernels/gl_spmv.cuh:25-100, and k_band merges the five descriptor interpreters
 // k_interp_band / k_band_causal_id / k_band_causal_c2 / k_band_embed / k_band_rope_x of
 // prover/cuda_primitives.py:605-734 behind a `kind` switch, keeping their arithmetic and names.
+#include <cooperative_groups.h>
+
 #include "../../include/verinf_b200.h"
 #include "blake3.cuh"
 #include "common.cuh"
 #include "gl.cuh"
+#include "gl3.cuh"
 
 namespace {
 
@@ -186,22 +189,38 @@ __global__ void __launch_bounds__(256, VI_MM_MINB) k_matmul(const uint64_t* __re
 
 // Thin product: M <= 4 rows of A against a tall B (k x n), out[mi][j] = sum_i A[mi][i] B[i][j].
 // This is the random linear combination of matrix rows (q_irs accumulation, prover/core.py:1351-1379;
-// combine_t, layergkr/gpu.py:301-308), which must stream B once: a CTA owns 32 columns, its 8 row
-// lanes take the rows i = lane, lane + 8, ... (every warp reads 256 contiguous bytes per row) with
-// unreduced 160-bit sums, and the 8 partial sums meet in shared memory.
+// combine_t, layergkr/gpu.py:301-308), which must stream B once: a CTA owns 32 columns, a warp reads 256
+// contiguous bytes per row, with unreduced 160-bit sums, and the 8 partial sums meet in shared memory.
+// What bounds it is how many loads are on the way: a matrix of a few thousand columns gives one CTA per SM at most, each
+// a chain of k / 8 loads.  So a cluster of up to 8 CTAs shares the rows of its 32 columns (partial sums meet through
+// distributed shared memory), and every warp has THIN_BATCH rows in flight: 1 x 1000 x 4096 54 -> 14 us.
+constexpr int THIN_BATCH = 4;
 template <int M>
 __global__ void __launch_bounds__(256) k_matmul_thin(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
                                                      uint64_t* __restrict__ C, int64_t k, int64_t n) {
-    __shared__ uint64_t red[8][M][32];
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int parts = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
+    __shared__ uint64_t red[8][M][32], sum[M][32];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t j = (int64_t)blockIdx.x * 32 + tx;
+    const int64_t j = (int64_t)(blockIdx.x / (unsigned)parts) * 32 + tx, step = 8 * parts;
     uint32_t acc[M][5];
 #pragma unroll
     for (int mi = 0; mi < M; ++mi)
 #pragma unroll
         for (int l = 0; l < 5; ++l) acc[mi][l] = 0;
     if (j < n) {
-        for (int64_t i = ty; i < k; i += 8) {
+        int64_t i = part * 8 + ty;
+        for (; i + (THIN_BATCH - 1) * step < k; i += THIN_BATCH * step) {
+            uint64_t b[THIN_BATCH];
+#pragma unroll
+            for (int u = 0; u < THIN_BATCH; ++u) b[u] = B[(i + u * step) * n + j];
+#pragma unroll
+            for (int u = 0; u < THIN_BATCH; ++u)
+#pragma unroll
+                for (int mi = 0; mi < M; ++mi) mac160(acc[mi], __ldg(A + mi * k + i + u * step), b[u]);
+        }
+        for (; i < k; i += step) {
             const uint64_t b = B[i * n + j];
 #pragma unroll
             for (int mi = 0; mi < M; ++mi) mac160(acc[mi], __ldg(A + mi * k + i), b);
@@ -210,18 +229,46 @@ __global__ void __launch_bounds__(256) k_matmul_thin(const uint64_t* __restrict_
 #pragma unroll
     for (int mi = 0; mi < M; ++mi) red[ty][mi][tx] = reduce160(acc[mi]);
     __syncthreads();
-    if (ty < M && j < n) {
+    if (ty < M) {
         uint64_t v = 0;
 #pragma unroll
         for (int r = 0; r < 8; ++r) v = add(v, red[r][ty][tx]);
+        sum[ty][tx] = v;
+    }
+    cluster.sync();
+    if (part == 0 && ty < M && j < n) {
+        uint64_t v = sum[ty][tx];
+        for (int q = 1; q < parts; ++q) v = add(v, *cluster.map_shared_rank(&sum[ty][tx], q));
         C[(int64_t)ty * n + j] = v;
     }
+    cluster.sync();             // no CTA leaves while another reads its sums
+}
+// CTAs per 32 columns: doubled while the grid stays within 8 CTAs per SM (what is resident at once) and a warp keeps a
+// batch of rows
+template <int M>
+int launch_thin(const uint64_t* A, const uint64_t* B, uint64_t* C, int64_t k, int64_t n, cudaStream_t st) {
+    const int64_t cols = (n + 31) / 32;
+    int64_t parts = 1;
+    while (parts < 8 && cols * parts * 2 <= 148 * 8 && k >= parts * 2 * 8 * THIN_BATCH) parts *= 2;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(cols * parts));
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)parts; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    VI_CUDA(cudaLaunchKernelEx(&cfg, k_matmul_thin<M>, A, B, C, k, n));
+    return vi::check_launch("k_matmul_thin");
 }
 
 // Weighted product column sum: part[s][j] = sum over the rows i of split s of
 // w[i] * EA[ia[i]][j] * EB[ib[i]][j].  One thread per column (coalesced rows), products summed
 // unreduced in five 32-bit limbs, one reduction per thread at the end; k_colsum_finish adds the
-// row splits (and the previous value when accumulating).
+// row splits (and the previous value when accumulating).  Bound by reading EA and EB once, which takes many loads on the
+// way: COLSUM_BATCH rows per thread and 16 CTAs per SM (1024 x 32768: 150 -> 111 us, 4.8 TB/s).
+constexpr int COLSUM_BATCH = 4;
 __global__ void __launch_bounds__(256) k_product_colsum(const uint64_t* __restrict__ EA, const uint64_t* __restrict__ EB,
                                                         int64_t n, const int64_t* __restrict__ ia,
                                                         const int64_t* __restrict__ ib, const uint64_t* __restrict__ w,
@@ -231,11 +278,22 @@ __global__ void __launch_bounds__(256) k_product_colsum(const uint64_t* __restri
     const int64_t i0 = (int64_t)blockIdx.y * rows_per_split;
     const int64_t i1 = i0 + rows_per_split < T ? i0 + rows_per_split : T;
     uint32_t x[5] = {0, 0, 0, 0, 0};
-    for (int64_t i = i0; i < i1; ++i) {
+    int64_t i = i0;
+    for (; i + COLSUM_BATCH <= i1; i += COLSUM_BATCH) {
+        uint64_t a[COLSUM_BATCH], b[COLSUM_BATCH];
+#pragma unroll
+        for (int u = 0; u < COLSUM_BATCH; ++u) {
+            a[u] = EA[(ia ? __ldg(ia + i + u) : i + u) * n + j];
+            b[u] = EB[(ib ? __ldg(ib + i + u) : i + u) * n + j];
+        }
+#pragma unroll
+        for (int u = 0; u < COLSUM_BATCH; ++u) mac160(x, w ? vg3::mul(a[u], __ldg(w + i + u)) : a[u], b[u]);
+    }
+    for (; i < i1; ++i) {
         const int64_t ra = ia ? __ldg(ia + i) : i, rb = ib ? __ldg(ib + i) : i;
         uint64_t a = EA[ra * n + j];
         const uint64_t b = EB[rb * n + j];
-        if (w) a = mul(a, __ldg(w + i));
+        if (w) a = vg3::mul(a, __ldg(w + i));
         mac160(x, a, b);
     }
     part[(int64_t)blockIdx.y * n + j] = reduce160(x);
@@ -250,19 +308,74 @@ __global__ void __launch_bounds__(256) k_colsum_finish(const uint64_t* __restric
     out[j] = v;
 }
 
-// w = M.v: one warp per row, lanes stride the row summing unreduced products, shuffle reduction.
+// w = M.v: WPR warps of a CTA per row, lanes stride the row summing unreduced products, shuffle reduction.
+// Bound by reading M once; MATVEC_BATCH entries per lane are on the way at a time, and rows are shared between warps
+// until the GPU is full of them.  PAIRS: rows and v start on 16-byte boundaries and two entries come with a load.
+// 4096 x 11008: 89 us with one warp per row and a load at a time, 75 us so (4.8 TB/s).
+constexpr int MATVEC_BATCH = 8;
+template <int WPR, bool PAIRS>
 __global__ void __launch_bounds__(256) k_matvec(const uint64_t* __restrict__ M, const uint64_t* __restrict__ v,
                                                 uint64_t* __restrict__ w, int64_t m, int64_t n) {
-    const int lane = threadIdx.x & 31;
-    const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (row >= m) return;
-    const uint64_t* r = M + row * n;
-    uint32_t x[5] = {0, 0, 0, 0, 0};
-    for (int64_t j = lane; j < n; j += 32) mac160(x, r[j], __ldg(v + j));
-    uint64_t acc = reduce160(x);
+    __shared__ uint64_t red[8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, in = wid % WPR;
+    const int64_t row = (int64_t)blockIdx.x * (8 / WPR) + wid / WPR;
+    uint64_t acc = 0;
+    if (row < m) {
+        const uint64_t* r = M + row * n;
+        uint32_t x[5] = {0, 0, 0, 0, 0};
+        constexpr int PER = PAIRS ? 2 : 1, STEP = 32 * WPR * PER, LOADS = MATVEC_BATCH / PER;
+        int64_t j = (32 * in + lane) * PER;
+        for (; j + (LOADS - 1) * STEP < n; j += LOADS * STEP) {          // with PAIRS n is even: j + 1 < n as well
+            if constexpr (PAIRS) {
+                ulonglong2 a[LOADS];
 #pragma unroll
-    for (int o = 16; o; o >>= 1) acc = add(acc, __shfl_xor_sync(0xffffffffu, acc, o));
-    if (lane == 0) w[row] = acc;
+                for (int u = 0; u < LOADS; ++u) a[u] = __ldcs(reinterpret_cast<const ulonglong2*>(r + j + u * STEP));
+#pragma unroll
+                for (int u = 0; u < LOADS; ++u) {
+                    const ulonglong2 b = __ldg(reinterpret_cast<const ulonglong2*>(v + j + u * STEP));
+                    mac160(x, a[u].x, b.x);
+                    mac160(x, a[u].y, b.y);
+                }
+            } else {
+                uint64_t a[LOADS];
+#pragma unroll
+                for (int u = 0; u < LOADS; ++u) a[u] = r[j + u * STEP];
+#pragma unroll
+                for (int u = 0; u < LOADS; ++u) mac160(x, a[u], __ldg(v + j + u * STEP));
+            }
+        }
+        for (; j < n; j += STEP) {
+            mac160(x, r[j], __ldg(v + j));
+            if (PAIRS) mac160(x, r[j + 1], __ldg(v + j + 1));
+        }
+        acc = reduce160(x);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) acc = add(acc, __shfl_xor_sync(0xffffffffu, acc, o));
+    }
+    if constexpr (WPR > 1) {
+        if (lane == 0) red[wid] = acc;
+        __syncthreads();
+        if (in != 0) return;
+#pragma unroll
+        for (int q = 1; q < WPR; ++q) acc = add(acc, red[wid + q]);
+    }
+    if (lane == 0 && row < m) w[row] = acc;
+}
+// Warps per row: doubled while all rows together leave room for them (64 warps per SM) and a warp keeps a whole batch.
+int launch_matvec(const uint64_t* M, const uint64_t* v, uint64_t* w, int64_t m, int64_t n, cudaStream_t st) {
+    int wpr = 1;
+    while (wpr < 8 && m * wpr * 2 <= 148 * 64 && n >= wpr * 2 * 32 * MATVEC_BATCH) wpr *= 2;
+    const int64_t grid = (m * wpr + 7) / 8;
+    VI_REQUIRE(grid <= 0x7FFFFFFFLL, "gl_matvec: too many rows");
+    const bool pairs = n % 2 == 0 && (((uintptr_t)M | (uintptr_t)v) & 15) == 0;
+    switch (wpr * 2 + pairs) {
+#define VI_CASE(x) \
+        case 2 * x: k_matvec<x, false><<<(unsigned)grid, 256, 0, st>>>(M, v, w, m, n); break; \
+        case 2 * x + 1: k_matvec<x, true><<<(unsigned)grid, 256, 0, st>>>(M, v, w, m, n); break;
+        VI_CASE(1) VI_CASE(2) VI_CASE(4) VI_CASE(8)
+#undef VI_CASE
+    }
+    return vi::check_launch("k_matvec");
 }
 
 __global__ void __launch_bounds__(BLOCK) k_spmv(const uint64_t* __restrict__ values, const uint64_t* __restrict__ col_idx,
@@ -441,19 +554,14 @@ extern "C" int vi_gl_matmul(const uint64_t* A, const uint64_t* B, uint64_t* C, i
     VI_REQUIRE(C != A && C != B, "gl_matmul: the output must not alias an input");
     VI_REQUIRE(k < (int64_t(1) << 32), "gl_matmul: inner dimension must be below 2^32");
     if (n == 1 && k > 0) {                     // a single column of B is a vector: matrix-vector product
-        int64_t g = (m * 32 + 255) / 256;
-        VI_REQUIRE(g <= 0x7FFFFFFFLL, "gl_matmul: too many rows");
-        k_matvec<<<(unsigned)g, 256, 0, (cudaStream_t)stream>>>(A, B, C, m, k);
-        return vi::check_launch("k_matvec");
+        return launch_matvec(A, B, C, m, k, (cudaStream_t)stream);
     }
     if (m <= 4 && k > 0 && (n + 31) / 32 <= 0x7FFFFFFFLL) {     // linear combination of the rows of B
-        const unsigned g = (unsigned)((n + 31) / 32);
         cudaStream_t st = (cudaStream_t)stream;
-        if (m == 1) k_matmul_thin<1><<<g, 256, 0, st>>>(A, B, C, k, n);
-        else if (m == 2) k_matmul_thin<2><<<g, 256, 0, st>>>(A, B, C, k, n);
-        else if (m == 3) k_matmul_thin<3><<<g, 256, 0, st>>>(A, B, C, k, n);
-        else k_matmul_thin<4><<<g, 256, 0, st>>>(A, B, C, k, n);
-        return vi::check_launch("k_matmul_thin");
+        if (m == 1) return launch_thin<1>(A, B, C, k, n, st);
+        if (m == 2) return launch_thin<2>(A, B, C, k, n, st);
+        if (m == 3) return launch_thin<3>(A, B, C, k, n, st);
+        return launch_thin<4>(A, B, C, k, n, st);
     }
     dim3 grid((unsigned)((n + MM_TN - 1) / MM_TN), (unsigned)((m + MM_TM - 1) / MM_TM));
     VI_REQUIRE(grid.y <= 65535, "gl_matmul: too many rows for one launch (m <= 4194240)");
@@ -465,10 +573,7 @@ extern "C" int vi_gl_matmul(const uint64_t* A, const uint64_t* B, uint64_t* C, i
 extern "C" int vi_gl_matvec(const uint64_t* M, const uint64_t* v, uint64_t* w, int64_t m, int64_t n, void* stream) {
     VI_REQUIRE(m >= 0 && n >= 0, "gl_matvec: negative size");
     if (m == 0) return VI_OK;
-    int64_t grid = (m * 32 + 255) / 256;
-    VI_REQUIRE(grid <= 0x7FFFFFFFLL, "gl_matvec: too many rows");
-    k_matvec<<<(unsigned)grid, 256, 0, (cudaStream_t)stream>>>(M, v, w, m, n);
-    return vi::check_launch("k_matvec");
+    return launch_matvec(M, v, w, m, n, (cudaStream_t)stream);
 }
 
 extern "C" int vi_gl_spmv(const uint64_t* values, const uint64_t* col_idx, const uint64_t* row_ptr,
@@ -511,21 +616,22 @@ extern "C" int vi_interp_band(int kind, uint64_t* out, int64_t out_off, int64_t 
 }
 
 namespace {
-int colsum_splits(int64_t T, int64_t n) {
-    // enough CTAs for ~4 per SM, at least 8 rows per split
+// row splits: per_sm CTAs per SM, at least 8 rows per split
+int colsum_splits(int64_t T, int64_t n, int per_sm) {
     int64_t col_blocks = (n + 255) / 256;
-    int64_t want = (148 * 4 + col_blocks - 1) / col_blocks;
+    int64_t want = (148 * per_sm + col_blocks - 1) / col_blocks;
     int64_t max_by_rows = (T + 7) / 8;
     int64_t s = want < max_by_rows ? want : max_by_rows;
     if (s < 1) s = 1;
     if (s > 1024) s = 1024;
     return (int)s;
 }
+constexpr int COLSUM_PER_SM = 16, COLSUM_PER_SM_LEAST = 4;      // with the recommended scratch / with less of it
 }  // namespace
 
 extern "C" int64_t vi_product_colsum_scratch_bytes(int64_t T, int64_t n) {
     if (T <= 0 || n <= 0) return 0;
-    return (int64_t)colsum_splits(T, n) * n * 8;
+    return (int64_t)colsum_splits(T, n, COLSUM_PER_SM) * n * 8;
 }
 
 extern "C" int vi_product_colsum(const uint64_t* EA, const uint64_t* EB, int64_t n,
@@ -541,10 +647,12 @@ extern "C" int vi_product_colsum(const uint64_t* EA, const uint64_t* EB, int64_t
     }
     VI_REQUIRE(EA && EB, "product_colsum: null input");
     VI_REQUIRE(T < (int64_t(1) << 32), "product_colsum: too many rows");
-    const int splits = colsum_splits(T, n);
-    if (scratch == nullptr || scratch_bytes < (int64_t)splits * n * 8)
+    const int least = colsum_splits(T, n, COLSUM_PER_SM_LEAST);
+    if (scratch == nullptr || scratch_bytes / (n * 8) < least)
         return vi::fail(VI_ERR_SCRATCH, "product_colsum: scratch of at least %lld bytes required (see vi_product_colsum_scratch_bytes)",
-                        (long long)((int64_t)splits * n * 8));
+                        (long long)((int64_t)least * n * 8));
+    int splits = colsum_splits(T, n, COLSUM_PER_SM);
+    if (scratch_bytes / (n * 8) < splits) splits = (int)(scratch_bytes / (n * 8));
     const int64_t per = (T + splits - 1) / splits;
     const int64_t gx = (n + 255) / 256;
     if (gx > 0x7FFFFFFFLL) return vi::fail(VI_ERR_LIMIT, "product_colsum: too many columns");
