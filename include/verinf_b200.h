@@ -161,10 +161,12 @@ int vi_merkle_level(const uint8_t* nodes, int64_t n_nodes, uint8_t* parents, voi
  * vi_product_colsum: out[j] (+)= sum_{i<T} w[i] * EA[ia[i]*n + j] * EB[ib[i]*n + j] for j < n;
  *   ia / ib (device int64, may be null = identity) select rows of the transformed matrices, so
  *   a row used by several constraints is transformed once; w (device, may be null = ones);
- *   accumulate != 0 adds into out.  scratch: vi_product_colsum_scratch_bytes(T, n). */
+ *   accumulate != 0 adds into out.  scratch: vi_product_colsum_scratch_bytes(T, n) at least;
+ *   up to vi_product_colsum_scratch_bytes_full(T, n) is used, for more row splits. */
 int vi_ntt_forward_padded(const uint64_t* src, int64_t m, int64_t k_in, uint64_t* dst, int64_t n,
                           void* scratch, int64_t scratch_bytes, void* stream);
 int64_t vi_product_colsum_scratch_bytes(int64_t T, int64_t n);
+int64_t vi_product_colsum_scratch_bytes_full(int64_t T, int64_t n);
 int vi_product_colsum(const uint64_t* EA, const uint64_t* EB, int64_t n,
                       const int64_t* ia_dev, const int64_t* ib_dev, const uint64_t* w_dev, int64_t T,
                       uint64_t* out, int accumulate, void* scratch, int64_t scratch_bytes, void* stream);

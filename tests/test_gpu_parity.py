@@ -664,7 +664,7 @@ def test_product_colsum_with_less_scratch(cp):
     T, n = 1003, 5000
     EA, EB, w = rnd_field(rng, (T, n)), rnd_field(rng, (T, n)), rnd_field(rng, T)
     a, b, wd = dev(EA), dev(EB), dev(w)
-    full, least = LIB.vi_product_colsum_scratch_bytes(T, n), 30 * n * 8       # 148 * 4 CTAs of 256 columns
+    full, least = LIB.vi_product_colsum_scratch_bytes_full(T, n), 30 * n * 8       # 148 * 4 CTAs of 256 columns
     outs = []
     for nb in (full, max(full - 8, least), least + 16, least):
         sc = torch.empty(nb, dtype=torch.uint8, device="cuda")

@@ -626,10 +626,14 @@ int colsum_splits(int64_t T, int64_t n, int per_sm) {
     if (s > 1024) s = 1024;
     return (int)s;
 }
-constexpr int COLSUM_PER_SM = 16, COLSUM_PER_SM_LEAST = 4;      // with the recommended scratch / with less of it
+constexpr int COLSUM_PER_SM = 16, COLSUM_PER_SM_LEAST = 4;      // with the full scratch / with the least
 }  // namespace
 
 extern "C" int64_t vi_product_colsum_scratch_bytes(int64_t T, int64_t n) {
+    if (T <= 0 || n <= 0) return 0;
+    return (int64_t)colsum_splits(T, n, COLSUM_PER_SM_LEAST) * n * 8;
+}
+extern "C" int64_t vi_product_colsum_scratch_bytes_full(int64_t T, int64_t n) {
     if (T <= 0 || n <= 0) return 0;
     return (int64_t)colsum_splits(T, n, COLSUM_PER_SM) * n * 8;
 }

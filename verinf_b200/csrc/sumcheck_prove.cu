@@ -18,6 +18,7 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "../../include/verinf_b200.h"
@@ -360,7 +361,8 @@ int take_slot(Slot** out) {
                 return VI_OK;
             }
     }
-    Slot* s = new Slot{dev, nullptr, nullptr, nullptr, 0};
+    Slot* s = new (std::nothrow) Slot{dev, nullptr, nullptr, nullptr, 0};
+    if (!s) return vi::fail(VI_ERR_CUDA, "sumcheck: out of host memory");
     cudaError_t e = cudaHostAlloc((void**)&s->host, SLOT_WORDS * 8, cudaHostAllocMapped | cudaHostAllocPortable);
     if (e == cudaSuccess) { memset(s->host, 0, SLOT_WORDS * 8); e = cudaHostGetDevicePointer((void**)&s->dev, s->host, 0); }
     if (e == cudaSuccess) e = cudaMalloc((void**)&s->ticket, 256);
@@ -606,7 +608,8 @@ extern "C" int vi_sumcheck_open(const uint64_t* const* tables, int n_tables, int
     if (work == nullptr || work_bytes < vi_sumcheck_session_work_bytes(n_tables, size))
         return vi::fail(VI_ERR_SCRATCH, "sumcheck: work buffer of at least %lld bytes required",
                         (long long)vi_sumcheck_session_work_bytes(n_tables, size));
-    Session* s = new Session{};
+    Session* s = new (std::nothrow) Session{};
+    if (!s) return vi::fail(VI_ERR_CUDA, "sumcheck: out of host memory");
     int rc = make_problem(s->pb, tables, n_tables, n_terms, coefs, nfac, fac);
     if (!rc) rc = take_slot(&s->slot);
     if (rc) { delete s; return rc; }

@@ -84,7 +84,7 @@ def product_colsum(EA, EB, weights=None, ia=None, ib=None, out=None):
     elif out.dtype != _U64 or out.numel() != n or not out.is_contiguous():
         raise RuntimeError("product_colsum: bad output tensor")
     with torch.cuda.device(EA.device):
-        nb = LIB.vi_product_colsum_scratch_bytes(T, n)
+        nb = LIB.vi_product_colsum_scratch_bytes_full(T, n)
         sc = scratch(nb, EA.device)
         check(LIB.vi_product_colsum(ptr(EA), ptr(EB), n, ptr(ia), ptr(ib), ptr(weights), T, ptr(out),
                                     1 if accumulate else 0, ptr(sc), nb, stream_ptr()))
