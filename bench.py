@@ -544,18 +544,15 @@ def run_native(a):
         dom_ms_per_step = dom[1][0] / a.steps
         achieved = bytes_per_step / (dom_ms_per_step * 1e-3) / 1e9 if dom_ms_per_step else 0.0
         enc_ms = sum(prof.get(t_, (0, 0))[0] for t_ in ("encode_pass1", "encode_mid", "encode_pass3")) / a.steps
-        # integer roofline of the encode: radix-16 butterfly element-stages and full modular multiplies at the
-        # warp-instruction counts of the field primitives measured with the integer-pipe microbenchmark
-        # (per element-stage 7.1 ALU-pipe + 4.7 FMA-pipe instructions, per multiply 15.1 + 13.8), against
-        # 148 SMs x 64 lanes per clock per pipe at the SM clock sampled during the run.  The ALU pipe is the
-        # fuller of the two; `issue_floor_ms` is the same work at the 128 lanes/clk/SM both pipes share.
+        # integer roofline of the encode: issue slots of its arithmetic, measured with the integer-pipe microbenchmark
+        # (a radix-16 butterfly 43 per element, 10.75 per radix-2 element-stage; a multiply 32), against 148 SMs x 4
+        # schedulers x 32 lanes per clock at the SM clock sampled during the run.  The coset twist is a multiply of
+        # its own only for blow-up factors other than 2 and 4.
         stages_per_row = (1 + a.blowup) * k * a.log_k
         muls_per_row = (1 + a.blowup) * k * 3 + a.blowup * k + k
-        alu_ops = rows * (stages_per_row * 7.1 + muls_per_row * 15.1)
-        all_ops = rows * (stages_per_row * 11.8 + muls_per_row * 29.3)
+        issue_muls = muls_per_row - (a.blowup * k if a.blowup in (2, 4) else 0)
         sm_hz = ((clocks or {}).get("sm_mhz") or 1965.0) * 1e6
-        alu_floor_ms = alu_ops / (148 * 64 * sm_hz) * 1e3
-        issue_floor_ms = all_ops / (148 * 128 * sm_hz) * 1e3
+        issue_floor_ms = rows * (stages_per_row * 10.75 + issue_muls * 32) / (148 * 128 * sm_hz) * 1e3
         # the two-term roofline the path's target is stated in: the slower of the bytes at the HBM peak and the
         # full modular multiplies at the measured multiply rate (855 G/s at 1965 MHz, integer-pipe microbenchmark);
         # butterflies, which are most of the work, are in neither term
@@ -571,8 +568,8 @@ def run_native(a):
                        "numa_bound": numa_bound,
                        "root": root_hex},
             # the fraction is of the HBM roofline (algorithmic bytes / time against the measured copy peak), as
-            # the metric asks; the kernel's limiter is integer-ALU issue, whose floor is `int_roofline`
-            "roofline": {"bound": "hbm", "limiter": "integer ALU issue (see int_roofline)", "kernel": dom[0],
+            # the metric asks; the kernel's limiter is integer issue, whose floor is `int_roofline`
+            "roofline": {"bound": "hbm", "limiter": "integer issue (see int_roofline)", "kernel": dom[0],
                          "achieved": achieved, "peak": hbm_peak,
                          "unit": "GB/s", "frac": achieved / hbm_peak, "peak_source": peak_src,
                          "traffic": (ncu_per_row[dom[0]] * rows * a.steps / dom[1][1]) if dom[0] in ncu_per_row else None,
@@ -587,11 +584,10 @@ def run_native(a):
             "encode_only": {"ms_per_step": enc_ms,
                             "gbs_algorithmic": rows * 8 * (k + n) / (enc_ms * 1e-3) / 1e9 if enc_ms else None,
                             "frac_of_hbm": rows * 8 * (k + n) / (enc_ms * 1e-3) / 1e9 / hbm_peak if enc_ms else None},
-            "int_roofline": {"bound": "integer ALU pipe (64 lanes/clk/SM)", "encode_floor_ms": alu_floor_ms,
-                             "issue_floor_ms": issue_floor_ms,
+            "int_roofline": {"bound": "integer issue slots (128 lanes/clk/SM)", "encode_floor_ms": issue_floor_ms,
                              "bytes_or_modmul_floor_ms": max(modmul_ms, bytes_ms), "modmul_floor_ms": modmul_ms,
                              "frac_of_bytes_or_modmul_floor": max(modmul_ms, bytes_ms) / enc_ms if enc_ms else None,
-                             "encode_ms": enc_ms, "frac": alu_floor_ms / enc_ms if enc_ms else None},
+                             "encode_ms": enc_ms, "frac": issue_floor_ms / enc_ms if enc_ms else None},
             "gpu_launches": launches,
             "clocks": clocks,
         }
