@@ -596,6 +596,31 @@ def test_whole_proofs_vs_oracle(logn, terms):
     assert all(np.array_equal(host(d), t) for d, t in zip(dts, tabs))
 
 
+@pytest.mark.parametrize("logn", [8, 13])
+@pytest.mark.parametrize("shape", _SHAPES + [[(1, [0, 1, 2, 3]), (P - 1, [4])], [(P - 1, [0, 1, 2, 3])]])
+def test_whole_proofs_of_small_signed_values(logn, shape):
+    """Tables of small signed numbers, as lifted int8 tensors have them: every pair of -4 .. 4 meets in a fold, so that the
+    line through a pair leaves [0, p) at each of the points where a round is summed."""
+    from verinf_b200 import layergkr_gpu as lg
+    nt = 1 + max(i for _, f in shape for i in f)
+    rng = np.random.default_rng(logn)
+    half = 1 << (logn - 1)
+    v = rng.integers(-128, 128, size=(nt, 2 * half))
+    pairs = np.array([(lo, hi) for lo in range(-4, 5) for hi in range(-4, 5)])
+    for t in v:
+        t[:81], t[half:half + 81] = rng.permutation(pairs).T
+    tabs = (v.astype(object) % P).astype(np.uint64)
+    coins = [int(c) for c in rnd_field(rng, logn)]
+    claim, samples, _ = oracle.sumcheck(tabs, shape, coins)
+    deg = max(len(f) for _, f in shape)
+    want = [[int(x) for x in row[:deg + 1]] for row in samples]
+    dts = [dev(t) for t in tabs]
+    plan = [(c, [dts[i] for i in f]) for c, f in shape]
+    for kw in (dict(), dict(coins=coins)):
+        got = lg.prove_terms_gpu(plan, lambda i: coins[i], **kw)
+        assert got[0] == claim and [[y for _, y in rp] for rp in got[1]] == want
+
+
 def test_whole_proofs_take_tables_as_before():
     """words of another 8-byte type, strided and 2-D tables, and a proof per thread and stream at once"""
     import threading

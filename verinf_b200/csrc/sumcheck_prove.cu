@@ -42,7 +42,7 @@ struct Terms {
     int n, deg;
     uint32_t count[MAX_TERMS];          // multiplicity of table k in bits 4k .. 4k+3
     int nfac[MAX_TERMS];
-    int sign[MAX_TERMS];                // coefficient 1, -1 (as sign) or general (0)
+    int sign[MAX_TERMS];                // coefficient 1, -1 (added or taken away as it is) or general (0)
     uint64_t coef[MAX_TERMS];
 };
 struct Tables { const uint64_t* in[MAX_TABLES]; uint64_t* out[MAX_TABLES]; };
@@ -71,15 +71,18 @@ __device__ __forceinline__ uint64_t add_any(uint64_t a, uint64_t m) {
 __device__ __forceinline__ uint64_t fold(uint64_t a, uint64_t b, uint64_t r) {
     return vg3::canon(add_any(a, vg3::mul(r, sub(b, a))));
 }
-// p - a for canonical a (p for 0): a word of the right residue
-__device__ __forceinline__ uint64_t neg_any(uint64_t a) { return vgl::P - a; }
 
-// Sum of words (three limbs) or of unreduced products (five limbs)
+// Sum of words (three limbs, the top one signed) or of unreduced products (five limbs)
 struct Acc {
     uint32_t x[5];
     __device__ __forceinline__ void clear() { x[0] = x[1] = x[2] = x[3] = x[4] = 0; }
     __device__ __forceinline__ void add_word(uint64_t v) {
         asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, 0;"
+            : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]) : "r"((uint32_t)v), "r"((uint32_t)(v >> 32)));
+    }
+    // a term with coefficient -1: words of any kind can be taken away, while p - v is a word only for v <= p
+    __device__ __forceinline__ void sub_word(uint64_t v) {
+        asm("sub.cc.u32 %0, %0, %3;\n\tsubc.cc.u32 %1, %1, %4;\n\tsubc.u32 %2, %2, 0;"
             : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]) : "r"((uint32_t)v), "r"((uint32_t)(v >> 32)));
     }
     __device__ __forceinline__ void add_product(uint64_t a, uint64_t b) {
@@ -88,7 +91,7 @@ struct Acc {
         asm("add.cc.u32 %0, %0, %5;\n\taddc.cc.u32 %1, %1, %6;\n\taddc.cc.u32 %2, %2, %7;\n\taddc.cc.u32 %3, %3, %8;\n\taddc.u32 %4, %4, 0;"
             : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]), "+r"(x[4]) : "r"(p0), "r"(p1), "r"(p2), "r"(p3));
     }
-    // [0, 2^64); 2^128 = -2^32, and fewer than 2^31 products are summed
+    // [0, 2^64); 2^128 = -2^32, and fewer than 2^31 words or products are summed
     __device__ __forceinline__ uint64_t value(bool products) const {
         if (!products) return vg3::norm3(T3{x[0], x[1], (int32_t)x[2]});
         const uint64_t r = vg3::reduce(x[0], x[1], x[2], x[3]);
@@ -118,10 +121,10 @@ __device__ __forceinline__ void add_point(Acc& acc, const uint64_t (&f)[NT], con
                 const uint32_t c = (tm.count[t] >> (4 * k)) & 15u;
                 for (uint32_t m = 0; m < c; ++m) {
                     if (have) p = vg3::mul(p, f[k]);
-                    else { p = sg < 0 ? neg_any(f[k]) : f[k]; have = true; }
+                    else { p = f[k]; have = true; }
                 }
             }
-            acc.add_word(p);
+            if (sg < 0) acc.sub_word(p); else acc.add_word(p);
         }
     }
 }
