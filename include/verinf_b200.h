@@ -258,7 +258,8 @@ int vi_sumcheck_complete(uint64_t* samples, int n_rounds, int deg, const uint64_
  *                       g(0) + g(1) is the claim.
  *   vi_sumcheck_open / _step / _close   one round per call: the first step gives round 0 (its r is ignored), every later
  *                       one folds with r, the challenge of the round before, and gives the next round's g(0..deg);
- *                       log2(size) steps in all.  A session is used by one thread at a time.
+ *                       log2(size) steps in all.  A session is used by one thread at a time, with the device current on
+ *                       which it was opened (a step on another one is refused).
  * work: device memory of vi_sumcheck_prove_work_bytes / vi_sumcheck_session_work_bytes bytes, 8-byte aligned, that
  * stays with the call or the session. */
 int64_t vi_sumcheck_prove_work_bytes(int n_tables, int64_t size);

@@ -175,3 +175,40 @@ def test_round_sample_derivation_host_logic():
     for k in range(1, 6):
         prev = [int(v) for v in samples[k - 1][:4]]
         assert (int(samples[k][0]) + int(samples[k][1])) % P == _interp_at(prev, coins[k - 1])
+
+
+def test_sumcheck_rounds_run_on_the_device_of_their_tables(monkeypatch):
+    """a callback may make another device current between two rounds: every call of a session, the first and the later ones,
+    is made inside the device of its tables"""
+    torch = pytest.importorskip("torch")
+    from verinf_b200 import layergkr_gpu as lg
+    inside, calls = [], []
+
+    class Device:
+        def __init__(self, dev):
+            self.dev = dev
+
+        def __enter__(self):
+            inside.append(self.dev)
+
+        def __exit__(self, *exc):
+            inside.pop()
+
+    class Lib:
+        def __getattr__(self, name):
+            def call(*args):
+                calls.append((name, list(inside)))
+                return 64 if name.endswith("_bytes") else 0
+            return call
+    monkeypatch.setattr(torch.cuda, "device", Device)
+    monkeypatch.setattr(lg, "LIB", Lib())
+    monkeypatch.setattr(lg, "stream_ptr", lambda: 0)
+    tables = [torch.zeros(8, dtype=torch.int64).view(torch.uint64) for _ in range(2)]
+    plan = lg._Plan(tables, [(1, [0, 1])])
+    for r in (None, 5, 7):
+        plan.round(r)
+    plan.run([1, 2, 3])
+    for name in ("vi_sumcheck_open", "vi_sumcheck_step", "vi_sumcheck_prove"):
+        got = [i for n, i in calls if n == name]
+        assert got and all(i == [tables[0].device] for i in got), (name, got)
+    assert not inside

@@ -47,6 +47,32 @@ dist.destroy_process_group()
 '''
 
 
+def test_sumcheck_session_stays_on_its_device():
+    """a callback that makes another device current changes nothing, and a step made on another device is refused"""
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs 2 GPUs")
+    import ctypes as C
+    from verinf_b200 import layergkr_gpu as lg
+    from verinf_b200._lib import LIB
+    tabs = [torch.arange(1, 65, dtype=torch.int64, device="cuda:0").view(torch.uint64) for _ in range(2)]
+
+    def coin(i):
+        torch.cuda.set_device(i % 2)
+        return 3 + i
+    with torch.cuda.device(0):
+        want = lg.prove_terms_gpu([(1, tabs)], lambda i: 3 + i)
+    with torch.cuda.device(0):
+        got = lg.prove_terms_gpu([(1, tabs)], coin)
+    assert got == want
+    with torch.cuda.device(0):
+        plan = lg._Plan(tabs, [(1, [0, 1])])
+        plan.round(None)
+    out = (C.c_uint64 * 8)()
+    with torch.cuda.device(1):
+        assert LIB.vi_sumcheck_step(plan._session, 3, out) == 1 and b"device 0" in LIB.vi_last_error()
+    plan.close()
+
+
 @pytest.mark.parametrize("world", [2, 4, 8])
 def test_sharded_commit_and_sumcheck_nccl(world, tmp_path):
     if torch.cuda.device_count() < world:

@@ -631,6 +631,9 @@ extern "C" int vi_sumcheck_step(void* session, uint64_t r, uint64_t* samples_hos
     VI_REQUIRE(!s->seen || r < vgl::P, "sumcheck: challenge not canonical");
     VI_REQUIRE(!s->seen || s->size >= 4, "sumcheck: no round left");
     Slot* slot = s->slot;
+    int dev;
+    VI_CUDA(cudaGetDevice(&dev));
+    VI_REQUIRE(dev == slot->device, "sumcheck: the session was opened on device %d, device %d is current", slot->device, dev);
     Sink sk{s->partials, slot->ticket, slot->dev, nullptr, slot->dev + (size_t)MAX_ROUNDS * ROW, ++slot->stamp};
     int rc = launch(s->pb, Launch{s->seen ? K_FOLD_ROUND : K_ROUND, s->size, r, 0, 0, nullptr}, sk, s->st);
     if (!rc) rc = wait_stamp(slot, s->st);

@@ -260,6 +260,7 @@ class _Plan:
                       (C.c_uint64 * n)(*[c for c, _ in terms]), (C.c_int32 * n)(*[len(f) for _, f in terms]),
                       (C.c_int32 * len(fac))(*fac))
         self._session = None
+        self._on = torch.cuda.device(self.dev)          # a session is tied to its device, whatever a callback makes current
 
     def _work(self, nbytes):
         return torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
@@ -269,7 +270,7 @@ class _Plan:
         n = len(coins)
         out = (C.c_uint64 * (8 * n))()
         nb = LIB.vi_sumcheck_prove_work_bytes(len(self.tables), self.size)
-        with torch.cuda.device(self.dev):
+        with self._on:
             work = self._work(nb)
             check(LIB.vi_sumcheck_prove(*self._args, (C.c_uint64 * n)(*coins), n, work.data_ptr(), nb, out, stream_ptr()))
         d = self.deg + 1
@@ -281,11 +282,12 @@ class _Plan:
             self._out = (C.c_uint64 * 8)()
             h = C.c_void_p()
             nb = LIB.vi_sumcheck_session_work_bytes(len(self.tables), self.size)
-            with torch.cuda.device(self.dev):
+            with self._on:
                 self._buf = self._work(nb)
                 check(LIB.vi_sumcheck_open(*self._args, self._buf.data_ptr(), nb, stream_ptr(), C.byref(h)))
             self._session = h
-        check(LIB.vi_sumcheck_step(self._session, r or 0, self._out))
+        with self._on:
+            check(LIB.vi_sumcheck_step(self._session, r or 0, self._out))
         return self._out[:self.deg + 1]
 
     def close(self):
