@@ -261,13 +261,16 @@ int vi_sumcheck_complete(uint64_t* samples, int n_rounds, int deg, const uint64_
  *                       log2(size) steps in all.  A session is used by one thread at a time, with the device current on
  *                       which it was opened (a step on another one is refused).
  * work: device memory of vi_sumcheck_prove_work_bytes / vi_sumcheck_session_work_bytes bytes, 8-byte aligned, that
- * stays with the call or the session. */
+ * stays with the call or the session.  A session reads the tables in its first two steps; with
+ * vi_sumcheck_session_work_bytes_own bytes of work the first step keeps a copy of them, and the caller may change or free
+ * them when it returns. */
 int64_t vi_sumcheck_prove_work_bytes(int n_tables, int64_t size);
 int vi_sumcheck_prove(const uint64_t* const* tables, int n_tables, int64_t size,
                       int n_terms, const uint64_t* coefs, const int32_t* nfac, const int32_t* fac,
                       const uint64_t* coins, int n_rounds, void* work, int64_t work_bytes,
                       uint64_t* samples_host, void* stream);
 int64_t vi_sumcheck_session_work_bytes(int n_tables, int64_t size);
+int64_t vi_sumcheck_session_work_bytes_own(int n_tables, int64_t size);
 int vi_sumcheck_open(const uint64_t* const* tables, int n_tables, int64_t size,
                      int n_terms, const uint64_t* coefs, const int32_t* nfac, const int32_t* fac,
                      void* work, int64_t work_bytes, void* stream, void** session);

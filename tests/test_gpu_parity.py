@@ -621,6 +621,30 @@ def test_whole_proofs_of_small_signed_values(logn, shape):
         assert got[0] == claim and [[y for _, y in rp] for rp in got[1]] == want
 
 
+@pytest.mark.parametrize("predraw", [False, True])
+@pytest.mark.parametrize("groups", [1, 3])
+@pytest.mark.parametrize("logn", [1, 2, 9, 12])
+def test_callbacks_may_write_to_the_tables(logn, groups, predraw):
+    """the proof is of the tables as they were at the call: one group of tables and several that share one, all challenges
+    drawn first and one per round"""
+    from verinf_b200 import layergkr_gpu as lg
+    rng = np.random.default_rng(logn + groups)
+    shape = [(1 + g, [0, 1 + g]) for g in range(1 if groups == 1 else 20)]
+    tabs = rnd_field(rng, (1 + len(shape), 1 << logn))
+    coins = [int(c) for c in rnd_field(rng, logn)]
+    want = lg.prove_terms_gpu([(c, [dev(tabs[i]) for i in f]) for c, f in shape], None, coins=coins)
+    if groups == 1:
+        claim, samples, _ = oracle.sumcheck(tabs, shape, coins)
+        assert want[0] == claim and [[y for _, y in rp] for rp in want[1]] == [[int(x) for x in row[:3]] for row in samples]
+    dts = [dev(t) for t in tabs]
+
+    def coin(i):
+        for d in dts:
+            d.view(torch.int64).add_(1 + i)
+        return coins[i]
+    assert lg.prove_terms_gpu([(c, [dts[i] for i in f]) for c, f in shape], coin, predraw=predraw) == want
+
+
 def test_whole_proofs_take_tables_as_before():
     """words of another 8-byte type, strided and 2-D tables, and a proof per thread and stream at once"""
     import threading

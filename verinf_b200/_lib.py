@@ -59,6 +59,7 @@ SIGNATURES = {
     "vi_sumcheck_prove_work_bytes": (_i64, [_int, _i64]),
     "vi_sumcheck_prove": (_int, [_p, _int, _i64, _int, _p, _p, _p, _p, _int, _p, _i64, _p, _p]),
     "vi_sumcheck_session_work_bytes": (_i64, [_int, _i64]),
+    "vi_sumcheck_session_work_bytes_own": (_i64, [_int, _i64]),
     "vi_sumcheck_open": (_int, [_p, _int, _i64, _int, _p, _p, _p, _p, _i64, _p, _p]),
     "vi_sumcheck_step": (_int, [_p, _u64, _p]),
     "vi_sumcheck_close": (_int, [_p]),

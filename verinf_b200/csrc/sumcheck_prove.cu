@@ -223,7 +223,8 @@ __device__ __forceinline__ void finish(const uint64_t (&v)[N], const Sink& sk) {
 }
 
 // ---- kernels ------------------------------------------------------------------------------------------------------
-// One round: FOLD = with the challenge r of the round before (size -> size/2, written to out), then the sums.
+// One round: FOLD = with the challenge r of the round before (size -> size/2, written to out, which may be in), then the
+// sums.  Without FOLD the entries are copied to out where there is one.
 template <int NT, bool SIMPLE, bool FOLD>
 __global__ void __launch_bounds__(BLOCK) k_round(Tables tb, Terms tm, int64_t size, uint64_t r, Sink sk) {
     const int64_t q = FOLD ? size / 4 : size / 2;
@@ -243,6 +244,10 @@ __global__ void __launch_bounds__(BLOCK) k_round(Tables tb, Terms tm, int64_t si
             } else {
                 lo[k] = f[i];
                 hi[k] = f[i + q];
+                if (tb.out[0]) {
+                    tb.out[k][i] = lo[k];
+                    tb.out[k][i + q] = hi[k];
+                }
             }
         }
         add_pair<NT, SIMPLE>(acc, lo, hi, tm, !FOLD);
@@ -527,6 +532,7 @@ struct Session {
     uint64_t *work, *partials;
     Slot* slot;
     cudaStream_t st;
+    bool own;                // the tables are copied by the first step and folded in place
     bool seen;
     uint64_t c[NPT];
 };
@@ -603,6 +609,10 @@ extern "C" int64_t vi_sumcheck_session_work_bytes(int n_tables, int64_t size) {
     if (n_tables <= 0 || size <= 0) return 0;
     return PARTIAL_BYTES + n_tables * (size / 2) * 8;
 }
+extern "C" int64_t vi_sumcheck_session_work_bytes_own(int n_tables, int64_t size) {
+    if (n_tables <= 0 || size <= 0) return 0;
+    return PARTIAL_BYTES + n_tables * size * 8;
+}
 
 extern "C" int vi_sumcheck_open(const uint64_t* const* tables, int n_tables, int64_t size, int n_terms, const uint64_t* coefs,
                                 const int32_t* nfac, const int32_t* fac, void* work, int64_t work_bytes, void* stream, void** session) {
@@ -619,7 +629,7 @@ extern "C" int vi_sumcheck_open(const uint64_t* const* tables, int n_tables, int
     s->size = size;
     s->partials = (uint64_t*)work;
     s->work = (uint64_t*)((char*)work + PARTIAL_BYTES);
-    for (int k = 0; k < n_tables; ++k) s->pb.tb.out[k] = s->work + k * (size / 2);
+    s->own = work_bytes >= vi_sumcheck_session_work_bytes_own(n_tables, size);
     s->st = (cudaStream_t)stream;
     *session = s;
     return VI_OK;
@@ -635,15 +645,17 @@ extern "C" int vi_sumcheck_step(void* session, uint64_t r, uint64_t* samples_hos
     VI_CUDA(cudaGetDevice(&dev));
     VI_REQUIRE(dev == slot->device, "sumcheck: the session was opened on device %d, device %d is current", slot->device, dev);
     Sink sk{s->partials, slot->ticket, slot->dev, nullptr, slot->dev + (size_t)MAX_ROUNDS * ROW, ++slot->stamp};
+    if (s->seen || s->own)      // from where the first launch that writes tables puts them, each stays in place
+        for (int k = 0; k < s->pb.nt; ++k)
+            if (!s->pb.tb.out[k]) s->pb.tb.out[k] = s->work + k * (s->own ? s->size : s->size / 2);
     int rc = launch(s->pb, Launch{s->seen ? K_FOLD_ROUND : K_ROUND, s->size, r, 0, 0, nullptr}, sk, s->st);
     if (!rc) rc = wait_stamp(slot, s->st);
     if (rc) return rc;
     const int deg = s->pb.tm.deg;
     round_poly(slot->host, deg, !s->seen, s->seen ? poly_at(s->c, deg, r) : 0, s->c, samples_host);
-    if (s->seen) {
-        s->size /= 2;
+    if (s->seen) s->size /= 2;
+    if (s->seen || s->own)
         for (int k = 0; k < s->pb.nt; ++k) s->pb.tb.in[k] = s->pb.tb.out[k];
-    }
     s->seen = true;
     return VI_OK;
 }

@@ -243,7 +243,7 @@ _MAX_TABLES, _MAX_TERMS = 8, 8          # per launch of the sumcheck kernels (cs
 
 
 class _Plan:
-    """Up to _MAX_TABLES tables (1-D uint64 CUDA tensors, read in place) and _MAX_TERMS terms as the C ABI takes them."""
+    """Up to _MAX_TABLES tables (1-D uint64 CUDA tensors, read where they are) and _MAX_TERMS terms as the C ABI takes them."""
 
     def __init__(self, tables: Sequence[torch.Tensor], terms: Sequence):
         self.tables, self.dev, self.size = tables, tables[0].device, tables[0].numel()
@@ -281,7 +281,7 @@ class _Plan:
         if self._session is None:
             self._out = (C.c_uint64 * 8)()
             h = C.c_void_p()
-            nb = LIB.vi_sumcheck_session_work_bytes(len(self.tables), self.size)
+            nb = LIB.vi_sumcheck_session_work_bytes_own(len(self.tables), self.size)     # the callback may write to the tables
             with self._on:
                 self._buf = self._work(nb)
                 check(LIB.vi_sumcheck_open(*self._args, self._buf.data_ptr(), nb, stream_ptr(), C.byref(h)))
@@ -394,7 +394,9 @@ def prove_terms_gpu(terms, coin: Callable[[int], int], field_p: int = P, mask=No
     interface implies (the callback receives nothing else, layergkr/gpu.py:402) and its call sites do
     (layergkr/relations.py:122-123 draws all challenges from the transcript, then passes
     `lambda i: coins[i]`).  The mask of a zero-knowledge proof only touches the scalar samples
-    (layergkr/gpu.py:392-396), so masked proofs are queued too."""
+    (layergkr/gpu.py:392-396), so masked proofs are queued too.
+
+    The proof is of the tables as they are at the call, whatever the callbacks write to them; no table is written."""
     assert field_p == P
     uniq, index, plan = [], {}, []
     for c, fs in terms:
@@ -407,9 +409,13 @@ def prove_terms_gpu(terms, coin: Callable[[int], int], field_p: int = P, mask=No
             idx.append(index[key])
         plan.append((c % P, idx))
     rows = []
+    draws = coins is None and predraw
     for f in uniq:
         if isinstance(f, torch.Tensor):
+            at = f.data_ptr()
             f = f.to(device="cuda").reshape(-1)
+            if draws and f.data_ptr() == at:  # coin() is called before the tables are read, and may write to them
+                f = f.clone()
             if f.dtype != torch.uint64:       # the words of another type, eight bytes each
                 f = f.view(torch.int64).view(torch.uint64)
             rows.append(f.contiguous())
