@@ -212,3 +212,9 @@ def test_sumcheck_rounds_run_on_the_device_of_their_tables(monkeypatch):
         got = [i for n, i in calls if n == name]
         assert got and all(i == [tables[0].device] for i in got), (name, got)
     assert not inside
+
+
+def test_built_code_depends_on_the_sources_alone():
+    """a compilation split over the processors that are free comes out differently each time, registers and spills included"""
+    from verinf_b200 import build
+    assert not [f for f in build.NVCC_FLAGS if f.startswith(("--split-compile", "-split-compile"))]
