@@ -106,6 +106,21 @@ def test_ntt_batched_vs_oracle(cp, logn, m):
     assert np.array_equal(host(y), oracle.ntt_batched(a, invert=True))
 
 
+@pytest.mark.parametrize("logn", range(1, 7))
+def test_ntt_short_tiles(cp, logn):
+    """transforms shorter than 128 points, whose tiles take the batch's width: batches around each power of two that a tile's
+    width can be, and around two of the widest tiles"""
+    rng = np.random.default_rng(50 + logn)
+    for width in (16, 32, 64, 128, 256, 512, 1024):
+        for m in (width - 1, width, width + 1):
+            a = rnd_field(rng, (m, 1 << logn))
+            x = dev(a)
+            cp.ntt_forward_batched(x)
+            assert np.array_equal(host(x), oracle.ntt_batched(a)), m
+            cp.ntt_inverse_batched(x)
+            assert np.array_equal(host(x), a), m
+
+
 @pytest.mark.parametrize("logn,m", [(25, 2), (26, 1)])
 def test_ntt_three_pass(cp, logn, m):
     """Lengths above 2^24 (three tile passes, split four-step factor tables; the reference's dispatch

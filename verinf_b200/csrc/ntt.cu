@@ -174,13 +174,18 @@ struct PassArgs {
 
 // Minimum resident CTAs per SM asked of the compiler for the 256-thread tiles (register budget =
 // 65536 / (256 * blocks)).  The passes are bound by instruction issue and hold 48 data registers in a radix-16
-// butterfly.  Measured (4096 rows, K = 2^16, 2 / 3 / 4 / 5 blocks where taken): plain first pass 1.48 ms at 3, 1.55 at 4
-// (which spills 16 bytes); with the pad PRG or the K-quant lift in its loader 4 is 1-4 % better; last pass 4.59 at 3,
-// 4.11 at 4, 15 % worse at 5; middle pass 6.80 at 2, 6.65 at 3.
+// butterfly.  Measured per tile length:
+//  * 128 and 256 points (4096 rows, K = 2^16): plain first pass 1.48 ms at 3, 1.55 at 4 (which spills 16 bytes); with the
+//    pad PRG or the K-quant lift in its loader 4 is 1-4 % better; last pass 4.59 at 3, 4.11 at 4, 15 % worse at 5; middle
+//    pass with shift twists 6.80 at 2, 6.65 at 3.
+//  * 16 to 64 points, 2^24 values (encodes: 2^25), us at 3 / 4 / 5 for the single pass: 2^4 53 / 51 / 57, 2^6 75 / 73 / 77;
+//    first and middle pass at 4 and 2 / 3 and 3: K = 2^9 x 4 267 / 271, K = 2^10 x 4 349 / 353, K = 2^12 x 4 377 / 378.
+//  * the middle pass with a twist table (blow-up 8 and others) keeps two register sets of 16 across the cosets: at 3 it
+//    spills 130-230 bytes.  K = 2^14 x 8 359 us at 2, 365 at 3, 390 at 1; K = 2^16 x 8 381, 388, 412; K = 2^10 x 8 337, 361, 362.
 constexpr int pass_min_ctas(int logl, int mode, int ld) {
-    return logl < 4 || logl > 8 ? 1 : mode == 0 && (ld == 0 || ld == 3) ? 3 : 4;
+    return logl < 4 || logl > 8 ? 1 : logl > 6 && mode == 0 && (ld == 0 || ld == 3) ? 3 : 4;
 }
-constexpr int mid_min_ctas(int logl) { return logl < 4 || logl > 8 ? 1 : 3; }
+constexpr int mid_min_ctas(int logl, int rho) { return logl < 4 || logl > 8 ? 1 : logl < 7 || rho == 0 ? 2 : 3; }
 // Columns per tile: fixed by the tile length from 128 points up (so that all tile index arithmetic is
 // compile-time), chosen by the host from the column count below that (tile_logC on the host).
 __host__ __device__ constexpr int fixed_logC(int logl) { return logl < 7 ? -1 : logl == 7 ? 5 : logl <= 9 ? 4 : 13 - logl; }
@@ -189,7 +194,8 @@ __host__ __device__ constexpr int fixed_logC(int logl) { return logl < 7 ? -1 : 
 __host__ __device__ constexpr int tile_max_threads(int logl) { return (logl >= 4 && logl <= 8) ? 256 : 512; }
 
 // Tile of C columns that lie one after the other in memory (L values each) into shared memory, sm[idx*CP + column];
-// columns from `valid` on are zero.
+// columns from `valid` on are zero.  Every thread has its EPT loads on the way at once: a loop of one load and one store a
+// turn took 98 us instead of 51 for 2^20 transforms of 16 points, 112 instead of 74 for 2^18 of 64.
 template <int LOGL>
 __device__ __forceinline__ void load_tile(uint64_t* sm, const uint64_t* __restrict__ src, int CP, int valid, int C) {
     constexpr int L = 1 << LOGL, LC = fixed_logC(LOGL);
@@ -203,6 +209,13 @@ __device__ __forceinline__ void load_tile(uint64_t* sm, const uint64_t* __restri
             if (L > NT) d[(i % PER) * NT * CP + i / PER] = src[tid + i * NT];
             else d[i * (NT >> LOGL)] = src[tid + i * NT];
         }
+    } else if (LC < 0) {
+        // tiles below 128 points, 16 columns or more: blockDim.x is a multiple of L, so all values of a thread share an index
+        constexpr int EPT = L < 16 ? L : 16;
+        const int nt = blockDim.x, step = nt >> LOGL, c0 = tid >> LOGL;
+        uint64_t* d = sm + (tid & (L - 1)) * CP + c0;
+#pragma unroll
+        for (int i = 0; i < EPT; ++i) d[i * step] = c0 + i * step < valid ? src[tid + i * nt] : 0;
     } else {
         for (int e = tid; e < L * C; e += blockDim.x) {
             const int idx = e & (L - 1), cl = e >> LOGL;
@@ -343,6 +356,12 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), pass_min_ctas(LOGL, MO
 #pragma unroll
             for (int i = 0; i < 16; ++i)
                 dst[tid + i * NT] = sm[(k0 + (i % PER) * NT) * CP + c0 + (L > NT ? i / PER : i * (NT >> LOGL))];
+        } else if (LC < 0) {
+            const int nt = blockDim.x, step = nt >> LOGL, c0 = tid >> LOGL;
+            const uint64_t* s = sm + (tid & (L - 1)) * CP + c0;
+#pragma unroll
+            for (int i = 0; i < EPT; ++i)
+                if (c0 + i * step < ncols_tile) dst[tid + i * nt] = s[i * step];
         } else {
             for (int e = tid; e < L * ncols_tile; e += blockDim.x) dst[e] = sm[(e & (L - 1)) * CP + (e >> LOGL)];
         }
@@ -448,7 +467,7 @@ __device__ __forceinline__ void coset_first(const uint64_t* __restrict__ c, int 
 // w_N^(t*l2) (folded into the four-step factor table), w_{RHO L}^(t*w) (folded into the stage-0
 // twiddle) and w_{16 RHO}^(t*j), a power of two applied as a shift: no twist multiply remains.
 template <int LOGL, int RHO>
-__global__ void __launch_bounds__(tile_max_threads(LOGL), mid_min_ctas(LOGL)) k_encode_mid(MidArgs a) {
+__global__ void __launch_bounds__(tile_max_threads(LOGL), mid_min_ctas(LOGL, RHO)) k_encode_mid(MidArgs a) {
     using SI = Sched<LOGL, false>;   // inverse: small stage first, radix-16 last
     using SF = Sched<LOGL, true>;    // forward: radix-16 first, small stage last
     constexpr int L = 1 << LOGL, EPT = SI::EPT;
@@ -506,9 +525,10 @@ __global__ void __launch_bounds__(tile_max_threads(LOGL), mid_min_ctas(LOGL)) k_
         }
     } else {
         // c2[j] = coefficient l1 = w + first_off(j) (held in c[brev(j)]) times K^-1 7^l, l = l1*n1 + l2; kept in
-        // shared memory behind the tile, element j of thread tid at c2[j * blockDim.x + tid]
+        // shared memory behind the tile, element j of thread tid at c2[j * nthr] (a compile-time stride
+        // from 128 points up: 215.3 -> 211.4 us for 128 rows of 2^16)
         uint64_t* c2 = sm + (size_t)L * CP + tid;
-        const int nthr = blockDim.x;
+        const int nthr = fixed_logC(LOGL) >= 0 ? (L / 16) << fixed_logC(LOGL) : (int)blockDim.x;
         const uint64_t* cs = a.cscale + colg + (int64_t)w * n1;
         const uint64_t* fs = a.fsN + colg + (int64_t)w * RHO * n1;
 #pragma unroll
