@@ -721,6 +721,16 @@ def test_thin_product_clusters(cp, k, n):
         assert np.array_equal(host(cp.gl_matmul(dev(A), dev(B))), oracle.gl_matmul(A, B))
 
 
+@pytest.mark.parametrize("m", [1, 2, 3, 4])
+@pytest.mark.parametrize("k,n", [(130, 9473), (130, 11840), (97, 18945), (33, 38001)])
+def test_thin_product_without_cluster(cp, m, k, n):
+    """column blocks around the counts from which a block has no cluster: 148 SMs times the CTAs resident on each"""
+    rng = np.random.default_rng(m + k + n)
+    A, B = rnd_field(rng, (m, k)), rnd_field(rng, (k, n))
+    A[:, 0], B[0] = P - 1, P - 1
+    assert np.array_equal(host(cp.gl_matmul(dev(A), dev(B))), oracle.gl_matmul(A, B))
+
+
 def test_product_colsum_with_less_scratch(cp):
     """the row splits follow the scratch that is there, down to what earlier callers were asked for"""
     from verinf_b200._lib import LIB, check, ptr, stream_ptr

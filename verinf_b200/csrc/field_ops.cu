@@ -193,14 +193,22 @@ __global__ void __launch_bounds__(256, VI_MM_MINB) k_matmul(const uint64_t* __re
 // contiguous bytes per row, with unreduced 160-bit sums, and the 8 partial sums meet in shared memory.
 // What bounds it is how many loads are on the way: a matrix of a few thousand columns gives one CTA per SM at most, each
 // a chain of k / 8 loads.  So a cluster of up to 8 CTAs shares the rows of its 32 columns (partial sums meet through
-// distributed shared memory), and every warp has THIN_BATCH rows in flight: 1 x 1000 x 4096 54 -> 14 us.
+// distributed shared memory), and every warp has THIN_BATCH rows in flight: 1 x 1000 x 4096 41 -> 17 us (cold L2).
+// Without a cluster (CLUSTER false) there are CTAs enough, and the loop of one row a turn, which the compiler unrolls, is
+// the faster one except for two rows of A: 1000 x 28672 at 1 / 2 / 3 / 4 rows 60 / 139 / 107 / 134 us, batched 70 / 103 / 139 / 153.
 constexpr int THIN_BATCH = 4;
-template <int M>
-__global__ void __launch_bounds__(256) k_matmul_thin(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
+// CTAs per SM asked of the compiler (0: its own choice): with 44 and 56 registers instead of the 48 and 64 that these leave,
+// it waits for each row's loads (4 x 4096 x 5000 267 us, 150 so)
+constexpr int thin_min_ctas(int m, bool cluster) { return !cluster || m == 1 ? 0 : m < 4 ? 5 : 4; }
+template <int M, bool CLUSTER>
+__global__ void __launch_bounds__(256, thin_min_ctas(M, CLUSTER)) k_matmul_thin(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
                                                      uint64_t* __restrict__ C, int64_t k, int64_t n) {
     namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    const int parts = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
+    int parts = 1, part = 0;
+    if constexpr (CLUSTER) {
+        parts = (int)cg::this_cluster().num_blocks();
+        part = (int)cg::this_cluster().block_rank();
+    }
     __shared__ uint64_t red[8][M][32], sum[M][32];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t j = (int64_t)(blockIdx.x / (unsigned)parts) * 32 + tx, step = 8 * parts;
@@ -211,14 +219,16 @@ __global__ void __launch_bounds__(256) k_matmul_thin(const uint64_t* __restrict_
         for (int l = 0; l < 5; ++l) acc[mi][l] = 0;
     if (j < n) {
         int64_t i = part * 8 + ty;
-        for (; i + (THIN_BATCH - 1) * step < k; i += THIN_BATCH * step) {
-            uint64_t b[THIN_BATCH];
+        if constexpr (CLUSTER || M == 2) {
+            for (; i + (THIN_BATCH - 1) * step < k; i += THIN_BATCH * step) {
+                uint64_t b[THIN_BATCH];
 #pragma unroll
-            for (int u = 0; u < THIN_BATCH; ++u) b[u] = B[(i + u * step) * n + j];
+                for (int u = 0; u < THIN_BATCH; ++u) b[u] = B[(i + u * step) * n + j];
 #pragma unroll
-            for (int u = 0; u < THIN_BATCH; ++u)
+                for (int u = 0; u < THIN_BATCH; ++u)
 #pragma unroll
-                for (int mi = 0; mi < M; ++mi) mac160(acc[mi], __ldg(A + mi * k + i + u * step), b[u]);
+                    for (int mi = 0; mi < M; ++mi) mac160(acc[mi], __ldg(A + mi * k + i + u * step), b[u]);
+            }
         }
         for (; i < k; i += step) {
             const uint64_t b = B[i * n + j];
@@ -229,27 +239,37 @@ __global__ void __launch_bounds__(256) k_matmul_thin(const uint64_t* __restrict_
 #pragma unroll
     for (int mi = 0; mi < M; ++mi) red[ty][mi][tx] = reduce160(acc[mi]);
     __syncthreads();
+    uint64_t v = 0;
     if (ty < M) {
-        uint64_t v = 0;
 #pragma unroll
         for (int r = 0; r < 8; ++r) v = add(v, red[r][ty][tx]);
-        sum[ty][tx] = v;
     }
-    cluster.sync();
-    if (part == 0 && ty < M && j < n) {
-        uint64_t v = sum[ty][tx];
-        for (int q = 1; q < parts; ++q) v = add(v, *cluster.map_shared_rank(&sum[ty][tx], q));
-        C[(int64_t)ty * n + j] = v;
+    if constexpr (CLUSTER) {
+        cg::cluster_group cluster = cg::this_cluster();
+        if (ty < M) sum[ty][tx] = v;
+        cluster.sync();
+        if (part == 0 && ty < M)
+            for (int q = 1; q < parts; ++q) v = add(v, *cluster.map_shared_rank(&sum[ty][tx], q));
+        cluster.sync();             // no CTA leaves while another reads its sums
     }
-    cluster.sync();             // no CTA leaves while another reads its sums
+    if (part == 0 && ty < M && j < n) C[(int64_t)ty * n + j] = v;
 }
-// CTAs per 32 columns: doubled while the grid stays within 8 CTAs per SM (what is resident at once) and a warp keeps a
-// batch of rows
+// CTAs per 32 columns: doubled while all clusters are resident at once (8, 5, 5 and 4 CTAs per SM at 1 .. 4 rows: registers)
+// and a warp keeps a batch of rows.  Clusters that have to wait for room cost far more than they bring: 3 x 4096 x 11008 in
+// pairs 447 us where 4 CTAs fit, 187 where 5 do.
 template <int M>
 int launch_thin(const uint64_t* A, const uint64_t* B, uint64_t* C, int64_t k, int64_t n, cudaStream_t st) {
+    static const int per_sm = [] {
+        int c = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_matmul_thin<M, true>, 256, 0) == cudaSuccess ? c : 0;
+    }();
     const int64_t cols = (n + 31) / 32;
     int64_t parts = 1;
-    while (parts < 8 && cols * parts * 2 <= 148 * 8 && k >= parts * 2 * 8 * THIN_BATCH) parts *= 2;
+    while (parts < 8 && cols * parts * 2 <= 148 * per_sm && k >= parts * 2 * 8 * THIN_BATCH) parts *= 2;
+    if (parts == 1) {
+        k_matmul_thin<M, false><<<(unsigned)cols, 256, 0, st>>>(A, B, C, k, n);
+        return vi::check_launch("k_matmul_thin");
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(cols * parts));
     cfg.blockDim = dim3(256);
@@ -259,7 +279,7 @@ int launch_thin(const uint64_t* A, const uint64_t* B, uint64_t* C, int64_t k, in
     at.val.clusterDim.x = (unsigned)parts; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    VI_CUDA(cudaLaunchKernelEx(&cfg, k_matmul_thin<M>, A, B, C, k, n));
+    VI_CUDA(cudaLaunchKernelEx(&cfg, k_matmul_thin<M, true>, A, B, C, k, n));
     return vi::check_launch("k_matmul_thin");
 }
 
