@@ -752,6 +752,26 @@ def test_product_colsum_with_less_scratch(cp):
     assert LIB.vi_product_colsum(ptr(a), ptr(b), n, None, None, ptr(wd), T, ptr(out), 0, ptr(sc), least - 8, stream_ptr()) != 0
 
 
+@pytest.mark.parametrize("T,n", [(1003, 3100), (385, 3200), (2048, 256), (24, 40000), (9, 1)])
+def test_product_colsum_splits(cp, T, n):
+    """row splits bounded by rows, by the columns, by the CTAs per SM and by their number, with the full and the least scratch"""
+    from verinf_b200 import fold
+    from verinf_b200._lib import LIB, check, ptr, stream_ptr
+    rng = np.random.default_rng(T + n)
+    EA, EB, w = rnd_field(rng, (T, n)), rnd_field(rng, (T, n)), rnd_field(rng, T)
+    EA[:, 0], EB[:, 0], w[0] = P - 1, P - 1, P - 1
+    a, b, wd = dev(EA), dev(EB), dev(w)
+    got = host(fold.product_colsum(a, b, wd))
+    nb = LIB.vi_product_colsum_scratch_bytes(T, n)
+    assert nb <= LIB.vi_product_colsum_scratch_bytes_full(T, n) <= max(nb, 48 * n * 8)
+    sc = torch.empty(nb, dtype=torch.uint8, device="cuda")
+    out = torch.zeros(n, dtype=torch.uint64, device="cuda")
+    check(LIB.vi_product_colsum(ptr(a), ptr(b), n, None, None, ptr(wd), T, ptr(out), 0, ptr(sc), nb, stream_ptr()))
+    assert np.array_equal(host(out), got)
+    for j in sorted({0, n // 2, n - 1}):
+        assert int(got[j]) == sum(int(x) * int(y) * int(z) for x, y, z in zip(w, EA[:, j], EB[:, j])) % P
+
+
 def test_linear_algebra(cp):
     rng = np.random.default_rng(5)
     A, B = rnd_field(rng, (37, 65)), rnd_field(rng, (65, 41))

@@ -287,7 +287,8 @@ int launch_thin(const uint64_t* A, const uint64_t* B, uint64_t* C, int64_t k, in
 // w[i] * EA[ia[i]][j] * EB[ib[i]][j].  One thread per column (coalesced rows), products summed
 // unreduced in five 32-bit limbs, one reduction per thread at the end; k_colsum_finish adds the
 // row splits (and the previous value when accumulating).  Bound by reading EA and EB once, which takes many loads on the
-// way: COLSUM_BATCH rows per thread and 16 CTAs per SM (1024 x 32768: 150 -> 111 us, 4.8 TB/s).
+// way: COLSUM_BATCH rows per thread and up to 16 CTAs per SM (1024 x 32768, cold L2: with
+// weights 160 -> 114 us, 4.7 TB/s; without 116 -> 106).
 constexpr int COLSUM_BATCH = 4;
 __global__ void __launch_bounds__(256) k_product_colsum(const uint64_t* __restrict__ EA, const uint64_t* __restrict__ EB,
                                                         int64_t n, const int64_t* __restrict__ ia,
@@ -636,26 +637,33 @@ extern "C" int vi_interp_band(int kind, uint64_t* out, int64_t out_off, int64_t 
 }
 
 namespace {
-// row splits: per_sm CTAs per SM, at least 8 rows per split
-int colsum_splits(int64_t T, int64_t n, int per_sm) {
-    int64_t col_blocks = (n + 255) / 256;
-    int64_t want = (148 * per_sm + col_blocks - 1) / col_blocks;
-    int64_t max_by_rows = (T + 7) / 8;
+// Row splits, at least 8 rows each: 4 CTAs per SM with the least scratch; with the full scratch up to 16, of at most
+// COLSUM_SPLITS splits, because k_colsum_finish adds a column's splits one after the other (us, cold L2, 4 CTAs per SM / 16 /
+// 16 of at most 48 splits: 2048 x 2048 38 / 48 / 33, 4000 x 1000 44 / 71 / 40, 2048 x 4096 52 / 56 / 46, 1024 x 32768
+// 159 / 115 / 114).
+constexpr int COLSUM_PER_SM = 16, COLSUM_PER_SM_LEAST = 4, COLSUM_SPLITS = 48;
+int colsum_splits(int64_t T, int64_t n, bool full) {
+    const int64_t col_blocks = (n + 255) / 256;
+    int64_t want = (148 * COLSUM_PER_SM_LEAST + col_blocks - 1) / col_blocks;
+    if (full && want < COLSUM_SPLITS) {
+        want = (148 * COLSUM_PER_SM + col_blocks - 1) / col_blocks;
+        if (want > COLSUM_SPLITS) want = COLSUM_SPLITS;
+    }
+    const int64_t max_by_rows = (T + 7) / 8;
     int64_t s = want < max_by_rows ? want : max_by_rows;
     if (s < 1) s = 1;
     if (s > 1024) s = 1024;
     return (int)s;
 }
-constexpr int COLSUM_PER_SM = 16, COLSUM_PER_SM_LEAST = 4;      // with the full scratch / with the least
 }  // namespace
 
 extern "C" int64_t vi_product_colsum_scratch_bytes(int64_t T, int64_t n) {
     if (T <= 0 || n <= 0) return 0;
-    return (int64_t)colsum_splits(T, n, COLSUM_PER_SM_LEAST) * n * 8;
+    return (int64_t)colsum_splits(T, n, false) * n * 8;
 }
 extern "C" int64_t vi_product_colsum_scratch_bytes_full(int64_t T, int64_t n) {
     if (T <= 0 || n <= 0) return 0;
-    return (int64_t)colsum_splits(T, n, COLSUM_PER_SM) * n * 8;
+    return (int64_t)colsum_splits(T, n, true) * n * 8;
 }
 
 extern "C" int vi_product_colsum(const uint64_t* EA, const uint64_t* EB, int64_t n,
@@ -671,11 +679,11 @@ extern "C" int vi_product_colsum(const uint64_t* EA, const uint64_t* EB, int64_t
     }
     VI_REQUIRE(EA && EB, "product_colsum: null input");
     VI_REQUIRE(T < (int64_t(1) << 32), "product_colsum: too many rows");
-    const int least = colsum_splits(T, n, COLSUM_PER_SM_LEAST);
+    const int least = colsum_splits(T, n, false);
     if (scratch == nullptr || scratch_bytes / (n * 8) < least)
         return vi::fail(VI_ERR_SCRATCH, "product_colsum: scratch of at least %lld bytes required (see vi_product_colsum_scratch_bytes)",
                         (long long)((int64_t)least * n * 8));
-    int splits = colsum_splits(T, n, COLSUM_PER_SM);
+    int splits = colsum_splits(T, n, true);
     if (scratch_bytes / (n * 8) < splits) splits = (int)(scratch_bytes / (n * 8));
     const int64_t per = (T + splits - 1) / splits;
     const int64_t gx = (n + 255) / 256;
