@@ -12,7 +12,7 @@
  *    process and never traps the device.
  *  - The only memory the library owns are immutable per-device twiddle tables,
  *    allocated (cudaMalloc + synchronous upload) the first time a transform
- *    length is used on a device, and up to 32 small result buffers (4 KB of mapped
+ *    length is used on a device, and up to 256 small result buffers (4 KB of mapped
  *    host memory each) per device that sumcheck proofs take turns with.
  *
  * Each declaration cites the reference interface it replaces (paths relative to

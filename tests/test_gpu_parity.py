@@ -660,6 +660,25 @@ def test_callbacks_may_write_to_the_tables(logn, groups, predraw):
     assert lg.prove_terms_gpu([(c, [dts[i] for i in f]) for c, f in shape], coin, predraw=predraw) == want
 
 
+def test_many_sessions_at_once():
+    """a proof of thousands of tables has hundreds of sessions open at once, more than the result buffers that are kept: equal
+    rounds from all of them, from the next ones, and after the buffers have been given back"""
+    from verinf_b200 import layergkr_gpu as lg
+    from verinf_b200._lib import LIB, check
+    rng = np.random.default_rng(8)
+    tabs = [dev(t) for t in rnd_field(rng, (2, 64))]
+    coins = [3, 5, 7, 9, 11, 13]
+    want = lg._Plan(tabs, [(1, [0, 1])]).run(coins)[:2]
+    for rep in range(3):
+        plans = [lg._Plan(tabs, [(1, [0, 1])]) for _ in range(260 if rep < 2 else 2)]
+        assert all(p.round(None) == want[0] for p in plans)
+        assert all(p.round(coins[0]) == want[1] for p in plans)
+        for p in plans:
+            p.close()
+        if rep == 1:
+            check(LIB.vi_release_tables())
+
+
 def test_whole_proofs_take_tables_as_before():
     """words of another 8-byte type, strided and 2-D tables, and a proof per thread and stream at once"""
     import threading

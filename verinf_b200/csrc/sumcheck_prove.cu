@@ -19,7 +19,6 @@
 #include <cstring>
 #include <mutex>
 #include <new>
-#include <vector>
 
 #include "../../include/verinf_b200.h"
 #include "common.cuh"
@@ -338,19 +337,22 @@ __global__ void __launch_bounds__(TAIL_BLOCK) k_tail(Tables tb, Terms tm, int si
 
 
 // ---- host side ----------------------------------------------------------------------------------------------------
-// Mapped host memory for the sums and a device word for the ticket, kept between proofs: at most SLOTS_KEPT per device,
-// each owned by one proof at a time; returned to the driver by release_slots().
+// Mapped host memory for the sums and a device word for the ticket, each owned by one proof at a time and kept between
+// proofs, at most SLOTS_KEPT idle ones per device: a proof of hundreds of tables has a session for every eight of them.
+// release_sumcheck_slots() returns them to the driver.  (In blocks of 32 the first 130 sessions took 424 ms instead of 49: a
+// pinned allocation of 100 KB takes far longer than 32 of 3 KB.)
 struct Slot {
     int device;
     uint64_t* host;          // MAX_ROUNDS rows, then the flag
     uint64_t* dev;           // its device address
     unsigned* ticket;
     uint64_t stamp;
+    Slot* next;              // in the list of idle ones
 };
 constexpr size_t SLOT_WORDS = (size_t)MAX_ROUNDS * ROW + 8;
-constexpr size_t SLOTS_KEPT = 32;
+constexpr int SLOTS_KEPT = 256;
 std::mutex g_slot_mu;
-std::vector<Slot*> g_slots;
+Slot* g_slots = nullptr;
 
 void free_slot(Slot* s) {
     cudaFreeHost(s->host);
@@ -362,14 +364,14 @@ int take_slot(Slot** out) {
     VI_CUDA(cudaGetDevice(&dev));
     {
         std::lock_guard<std::mutex> lk(g_slot_mu);
-        for (size_t i = 0; i < g_slots.size(); ++i)
-            if (g_slots[i]->device == dev) {
-                *out = g_slots[i];
-                g_slots.erase(g_slots.begin() + i);
+        for (Slot** at = &g_slots; *at; at = &(*at)->next)
+            if ((*at)->device == dev) {
+                *out = *at;
+                *at = (*at)->next;
                 return VI_OK;
             }
     }
-    Slot* s = new (std::nothrow) Slot{dev, nullptr, nullptr, nullptr, 0};
+    Slot* s = new (std::nothrow) Slot{dev, nullptr, nullptr, nullptr, 0, nullptr};
     if (!s) return vi::fail(VI_ERR_CUDA, "sumcheck: out of host memory");
     cudaError_t e = cudaHostAlloc((void**)&s->host, SLOT_WORDS * 8, cudaHostAllocMapped | cudaHostAllocPortable);
     if (e == cudaSuccess) { memset(s->host, 0, SLOT_WORDS * 8); e = cudaHostGetDevicePointer((void**)&s->dev, s->host, 0); }
@@ -388,9 +390,9 @@ int take_slot(Slot** out) {
 void give_slot(Slot* s) {
     {
         std::lock_guard<std::mutex> lk(g_slot_mu);
-        size_t n = 0;
-        for (Slot* o : g_slots) n += o->device == s->device;
-        if (n < SLOTS_KEPT) { g_slots.push_back(s); return; }
+        int n = 0;
+        for (Slot* o = g_slots; o; o = o->next) n += o->device == s->device;
+        if (n < SLOTS_KEPT) { s->next = g_slots; g_slots = s; return; }
     }
     free_slot(s);
 }
@@ -534,6 +536,7 @@ struct Session {
     cudaStream_t st;
     bool own;                // the tables are copied by the first step and folded in place
     bool seen;
+    bool failed;             // a launch may not have ended: the slot is not used again
     uint64_t c[NPT];
 };
 
@@ -542,8 +545,11 @@ struct Session {
 namespace vi {
 void release_sumcheck_slots() {
     std::lock_guard<std::mutex> lk(g_slot_mu);
-    for (Slot* s : g_slots) free_slot(s);
-    g_slots.clear();
+    while (g_slots) {
+        Slot* s = g_slots;
+        g_slots = s->next;
+        free_slot(s);
+    }
 }
 }  // namespace vi
 
@@ -650,7 +656,7 @@ extern "C" int vi_sumcheck_step(void* session, uint64_t r, uint64_t* samples_hos
             if (!s->pb.tb.out[k]) s->pb.tb.out[k] = s->work + k * (s->own ? s->size : s->size / 2);
     int rc = launch(s->pb, Launch{s->seen ? K_FOLD_ROUND : K_ROUND, s->size, r, 0, 0, nullptr}, sk, s->st);
     if (!rc) rc = wait_stamp(slot, s->st);
-    if (rc) return rc;
+    if (rc) { s->failed = true; return rc; }
     const int deg = s->pb.tm.deg;
     round_poly(slot->host, deg, !s->seen, s->seen ? poly_at(s->c, deg, r) : 0, s->c, samples_host);
     if (s->seen) s->size /= 2;
@@ -663,7 +669,7 @@ extern "C" int vi_sumcheck_step(void* session, uint64_t r, uint64_t* samples_hos
 extern "C" int vi_sumcheck_close(void* session) {
     if (!session) return VI_OK;
     Session* s = (Session*)session;
-    give_slot(s->slot);
+    if (!s->failed) give_slot(s->slot);
     delete s;
     return VI_OK;
 }
