@@ -139,6 +139,8 @@ __global__ void k_selfcheck(unsigned long long* bad) {
         const vg3::T3 t = vg3::sub3(vg3::widen(a), vg3::widen(b));
         const uint64_t d = sub(a, b);
         if (vg3::canon(vg3::norm3(vg3::shl3<12>(t))) != mul_pow2<12>(d) || vg3::canon(vg3::norm3(vg3::shl3<39>(t))) != mul_pow2<39>(d) ||
+            vg3::canon(vg3::norm3(vg3::shl3<32>(t))) != mul_pow2<32>(d) || vg3::canon(vg3::norm3(vg3::shl3<36>(t))) != mul_pow2<36>(d) ||
+            vg3::canon(vg3::norm3(vg3::shl3<48>(t))) != mul_pow2<48>(d) || vg3::canon(vg3::norm3(vg3::shl3<60>(t))) != mul_pow2<60>(d) ||
             vg3::canon(vg3::norm3(vg3::shl3<78>(t))) != mul_pow2<78>(d) || vg3::canon(vg3::norm3(vg3::shl3<96>(t))) != sub(0, d) ||
             vg3::canon(vg3::norm3(vg3::shl3<117>(t))) != sub(0, mul_pow2<21>(d)) ||
             vg3::canon(vg3::norm3(vg3::shl3<156>(t))) != sub(0, mul_pow2<60>(d)) ||
@@ -159,7 +161,7 @@ float time_ms(F launch) {
 }
 }  // namespace
 
-int main() {
+int main(int argc, char**) {      // any argument: the self-check alone
     void* d = nullptr;
     if (cudaMalloc(&d, (size_t)GRID * BLOCK * 8) != cudaSuccess) { printf("no CUDA device\n"); return 1; }
     {
@@ -169,6 +171,7 @@ int main() {
         printf("self-check of add/sub/mul/reduce128/mul_pow2 and the three-limb form vs 128-bit arithmetic: %s (flags %llu) %s\n",
                h ? "MISMATCH" : "ok", h, cudaGetErrorString(cudaGetLastError()));
         cudaFree(bad);
+        if (argc > 1) return h != 0 || cudaGetLastError() != cudaSuccess;
     }
     int khz = 0; cudaDeviceGetAttribute(&khz, cudaDevAttrClockRate, 0);
     const double threads = (double)GRID * BLOCK;

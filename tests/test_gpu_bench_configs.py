@@ -33,3 +33,13 @@ def test_bench_self_check_on_the_quoted_configurations():
     assert line["layer7b"]["sumcheck_claims_match_rho_Y_tau"] is True
     assert line["sharded_commit"]["root"] == line["config"]["root"]
     assert line["gpu_launches"] > 0 and line["roofline"]["frac"] > 0
+
+
+def test_field_primitives_against_128_bit_arithmetic():
+    """The self-check of the field primitives (bench_int_pipes.cu): sums, products, shifts and radix-16 DFTs in canonical and in
+    three-limb form at edges and at random words, the shifts by 32 .. 63 among them, whose carry chain counts on how the
+    assembler keeps the carry flag."""
+    sys.path.insert(0, str(ROOT))
+    import bench
+    p = subprocess.run([str(bench.build_int_pipes()), "check"], capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and ": ok (flags 0) no error" in p.stdout, p.stdout + p.stderr

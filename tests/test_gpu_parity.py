@@ -262,7 +262,8 @@ def test_encode_vs_oracle(cp, ell, k, n, m, pad):
                                    (1024, 4096, 70), (1024, 8192, 2), (2048, 8192, 9), (4096, 16384, 2), (8192, 65536, 1),
                                    (16384, 65536, 1), (16384, 32768, 37)])
 def test_encode_few_tiles(cp, k, n, m):
-    """too few tiles for the GPU: cosets of a tile dealt out to CTAs, tiles cut down to 16 columns; blow-ups 1 to 16"""
+    """batches of few tiles, from one to some thousand, at blow-ups 1 to 16: the shift twists (2 and 4) and the twist table
+    (others), tiles of 1 to 128 points with run-time and compile-time widths, full and partial ones"""
     rng = np.random.default_rng(k + n + m)
     msg = rnd_field(rng, (m, k))
     want_p, want_c = oracle.encode_rows(msg, n)
@@ -591,7 +592,8 @@ _SHAPES = [[(1, [0, 1])], [(1, [0, 1, 2])], [(1, [0])], [(1, [0, 1, 2, 3])], [(1
 @pytest.mark.parametrize("terms", range(len(_SHAPES)))
 def test_whole_proofs_vs_oracle(logn, terms):
     """Proofs from the caller's tables, challenges known and one at a time: product terms and general ones, sizes around
-    the one-block and the host rounds, entries 0 and p - 1 in the first pair of every table; tables left as they are."""
+    the one-block rounds (up to 2^11 entries) and the two-round passes, entries 0 and p - 1 in the first pair of every
+    table; tables left as they are."""
     from verinf_b200 import layergkr_gpu as lg
     shape = _SHAPES[terms]
     nt = 1 + max(i for _, f in shape for i in f)

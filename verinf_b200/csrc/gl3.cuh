@@ -165,11 +165,16 @@ __device__ __forceinline__ T3 shl3(T3 a) {
                 : "=&r"(r.x0), "=&r"(r.x1), "=&r"(r.x2) : "r"(l0), "r"(l1), "r"(l2), "r"(s));
             return r;
         } else if constexpr (U == 1 && !NEG) {  // l0 phi + l1 (phi - 1) - l2
+            // The one chain here that changes direction: madc reads the flag that subc.cc left.  PTX calls that flag the
+            // borrow; the assembler for sm_100a keeps one carry flag, set when there is NO borrow, and this counts on it (the
+            // -1 ahead stands for the borrow).  Nothing in the PTX document promises it: bench_int_pipes.cu checks it against
+            // 128-bit arithmetic, and every transform of 16 points and more against the oracle would be wrong without it.
+            // Both forms that stay inside the document are slower (last pass of the encode 3 and 4 %, middle pass 0.5 and 0.6 %).
             asm("{\n\t.reg .u32 e0, e1;\n\t.reg .b64 e;\n\t"
                 "mul.wide.u32 e, %4, %7;\n\t"
                 "mov.b64 {e0, e1}, e;\n\t"
                 "add.cc.u32 %1, e1, %3;\n\t"
-                "addc.u32 %2, 0xffffffff, 0;\n\t"      // carry - 1: the chain below ends with a carry, not a borrow
+                "addc.u32 %2, 0xffffffff, 0;\n\t"      // carry - 1
                 "sub.cc.u32 %0, e0, %5;\n\t"
                 "subc.cc.u32 %1, %1, %6;\n\t"
                 "madc.lo.u32 %2, %6, %7, %2;\n\t}"
