@@ -14,6 +14,133 @@
 #include "verinf_b200/csrc/dft_reg.cuh"
 #include "verinf_b200/csrc/gl.cuh"
 
+// The canonical form of the power-of-two shifts and of the in-register DFT, which the library had before gl3.cuh: what
+// the three-limb form is timed and checked against.
+namespace vgl {
+#ifdef __CUDA_ARCH__
+// (l1:l0) + h*(2^32-1) mod p, canonical; (l1:l0) is any u64, h any u32: 12 instructions
+__device__ __forceinline__ uint64_t add_mul_eps(uint32_t l0, uint32_t l1, uint32_t h) {
+    uint32_t r0, r1;
+#if VGL_FMA_CARRY & 4
+    asm("{\n\t.reg .u32 c, e0, e1;\n\t.reg .b64 e;\n\t.reg .pred q;\n\t"
+        "mul.wide.u32 e, %4, %5;\n\t"          // e = h*EPS (FMA pipe)
+        "mov.b64 {e0, e1}, e;\n\t"
+        "add.cc.u32 %0, %2, e0;\n\t"
+        "addc.cc.u32 %1, %3, e1;\n\t"
+        "addc.u32 c, 0, 0;\n\t"
+        "mad.lo.cc.u32 %0, c, %5, %0;\n\t"     // += carry ? EPS : 0 (FMA pipe)
+        "madc.lo.u32 %1, c, %6, %1;\n\t"
+        "setp.eq.u32 q, %1, 0xffffffff;\n\t"
+        "setp.ne.and.u32 q, %0, 0, q;\n\t"
+        "@q mov.u32 %1, 0;\n\t"
+        "@q add.u32 %0, %0, 0xffffffff;\n\t}"
+        : "=&r"(r0), "=&r"(r1) : "r"(l0), "r"(l1), "r"(h), "r"(VGL_M1), "r"(VGL_ZERO));
+    return pack(r0, r1);
+#endif
+    asm("{\n\t.reg .u32 m, e0, e1;\n\t.reg .pred q;\n\t"
+        "sub.cc.u32 e0, 0, %4;\n\t"
+        "subc.u32 e1, %4, 0;\n\t"
+        "add.cc.u32 %0, %2, e0;\n\t"
+        "addc.cc.u32 %1, %3, e1;\n\t"
+        "addc.u32 m, 0, 0;\n\t"
+        "neg.s32 m, m;\n\t"
+        "add.cc.u32 %0, %0, m;\n\t"
+        "addc.u32 %1, %1, 0;\n\t"
+        "setp.eq.u32 q, %1, 0xffffffff;\n\t"
+        "setp.ne.and.u32 q, %0, 0, q;\n\t"
+        "@q mov.u32 %1, 0;\n\t"
+        "@q add.u32 %0, %0, 0xffffffff;\n\t}"
+        : "=&r"(r0), "=&r"(r1) : "r"(l0), "r"(l1), "r"(h));
+    return pack(r0, r1);
+}
+#endif
+
+// x * 2^S mod p for a compile-time 0 <= S < 96 (x canonical -> canonical).
+// Every 2^k-th root of unity with k <= 6 is a power of two in this field
+// (2 has order 192), so radix-<=64 butterflies multiply by shifts only.
+// With phi = 2^32 (phi^2 = phi - 1, phi^3 = -1) and (l2:l1:l0) = x << (S mod 32):
+//   S <  32: (l1:l0) + l2*(2^32-1)
+//   S <  64: the general 128-bit reduction of (l2:l1:l0:0)
+//   S >= 64: l0*(2^32-1) - (l2:l1)
+// (Issuing the limb shifts as wide multiplies on the FMA pipe, or building the 64-bit sums from
+// mad.wide plus a 64-bit compare instead of carry chains, was measured slower on B200: radix-16
+// butterfly throughput 2004 and 1250 G element-stages/s against 2091 for this form.)
+template <int S>
+__device__ __forceinline__ uint64_t mul_pow2(uint64_t x) {
+    static_assert(S >= 0 && S < 96, "shift out of range");
+#ifdef __CUDA_ARCH__
+    if constexpr (S == 0) {
+        return x;
+    } else {
+        constexpr int V = S % 32, U = S / 32;
+        // (l2:l1:l0) = x << V as three 32-bit limbs
+        uint32_t l0 = (uint32_t)x, l1 = (uint32_t)(x >> 32), l2 = 0;
+        if constexpr (V != 0) {
+            l2 = l1 >> (32 - V); l1 = (l1 << V) | (l0 >> (32 - V)); l0 <<= V;
+        }
+        if constexpr (U == 0) {
+            // l0 + l1 phi + l2 phi^2 = (l1:l0) + l2*(2^32-1)
+            return add_mul_eps(l0, l1, l2);
+        } else if constexpr (U == 1) {
+            // l0 phi + l1 phi^2 + l2 phi^3: the 128-bit value (hi = (l2:l1), lo = (l0:0))
+            return reduce128(pack(0, l0), pack(l1, l2));
+        } else {
+            // l0 phi^2 + l1 phi^3 + l2 phi^4 = l0*(2^32-1) - (l2:l1); (l2:l1) < 2^63 is canonical
+#if VGL_FMA_CARRY & 4
+            uint64_t e;
+            asm("mul.wide.u32 %0, %1, %2;" : "=l"(e) : "r"(l0), "r"(VGL_M1));     // FMA pipe
+            return sub(e, pack(l1, l2));
+#else
+            uint32_t e0, e1;
+            asm("sub.cc.u32 %0, 0, %2;\n\t"
+                "subc.u32 %1, %2, 0;"
+                : "=&r"(e0), "=&r"(e1) : "r"(l0));
+            return sub(pack(e0, e1), pack(l1, l2));
+#endif
+        }
+    }
+#else
+    return x;
+#endif
+}
+
+}  // namespace vgl
+
+namespace vdft {
+
+using vgl::add;
+using vgl::sub;
+
+template <int LOGLEN, int K, bool INV>
+__device__ __forceinline__ void bfly(uint64_t& a, uint64_t& b) {
+    constexpr int s0 = (root_exp(LOGLEN) * K) % 192;
+    constexpr int s = INV ? (192 - s0) % 192 : s0;
+    uint64_t t = add(a, b);
+    uint64_t d = (s >= 96) ? sub(b, a) : sub(a, b);   // 2^96 = -1
+    a = t;
+    b = vgl::mul_pow2<s % 96>(d);
+}
+
+template <int LOGR, int LOGLEN, int I, bool INV>
+__device__ __forceinline__ void dif_level(uint64_t* v) {
+    constexpr int R = 1 << LOGR, LEN = 1 << LOGLEN, HALF = LEN / 2;
+    if constexpr (I < R / 2) {
+        constexpr int blk = I / HALF, k = I % HALF;
+        bfly<LOGLEN, k, INV>(v[blk * LEN + k], v[blk * LEN + k + HALF]);
+        dif_level<LOGR, LOGLEN, I + 1, INV>(v);
+    }
+}
+// In-register decimation-in-frequency DFT of R = 2^LOGR values: X[c] = v[bitrev(c)].
+template <int LOGR, int LOGLEN, bool INV>
+__device__ __forceinline__ void dif(uint64_t* v) {
+    if constexpr (LOGLEN >= 1) {
+        dif_level<LOGR, LOGLEN, 0, INV>(v);
+        dif<LOGR, LOGLEN - 1, INV>(v);
+    }
+}
+
+}  // namespace vdft
+
 namespace {
 constexpr int ITERS = 1024, CHAINS = 8, GRID = 148 * 8, BLOCK = 256;
 

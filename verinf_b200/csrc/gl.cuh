@@ -7,7 +7,8 @@
 //
 // The device versions are written on 32-bit limbs with explicit carry chains
 // (add.cc / subc): on sm_100a the integer ALU pipe and the FMA pipe each issue half a warp
-// per cycle and the NTT kernels are bound by them, so every op is the shortest sequence found
+// per cycle and the kernels that use them (element-wise ops, products, sharded sumchecks) are
+// bound by them, so every op is the shortest sequence found
 // (sub = 5 instructions, add = neg + sub = 7, reduce128 = 16) with its instructions spread
 // over both pipes (VGL_FMA_CARRY below).
 #pragma once
@@ -24,8 +25,10 @@ __host__ __device__ __forceinline__ uint64_t pack(uint32_t lo, uint32_t hi) { re
 // mad.lo.cc / madc.lo with a multiplier of 1, -1 or 0 taken from the constant bank (so that the assembler
 // keeps them multiply-adds).  With VGL_FMA_CARRY the conditional corrections of sub, reduce128 and the
 // power-of-two shifts (+-(2^32 - 1) after a borrow or carry) and the products h*(2^32 - 1) are issued that
-// way: the kernels built on these primitives are bound by the ALU pipe while the FMA pipe is a quarter busy.
-// Bits: 1 = the correction of sub, 2 = reduce128 (the tail of every full multiply), 4 = the power-of-two shifts.
+// way: kernels built on the other form are bound by the ALU pipe while the FMA pipe is a quarter busy.  The transforms and
+// whole sumcheck proofs use the unreduced forms of gl3.cuh.
+// Bits: 1 = the correction of sub, 2 = reduce128 (the tail of every full multiply), 4 = the power-of-two shifts of
+// bench_int_pipes.cu.
 #ifndef VGL_FMA_CARRY
 #define VGL_FMA_CARRY 7
 #endif
@@ -151,44 +154,6 @@ __host__ __device__ __forceinline__ uint64_t reduce128(uint64_t lo, uint64_t hi)
 #endif
 }
 
-#ifdef __CUDA_ARCH__
-// (l1:l0) + h*(2^32-1) mod p, canonical; (l1:l0) is any u64, h any u32: 12 instructions
-__device__ __forceinline__ uint64_t add_mul_eps(uint32_t l0, uint32_t l1, uint32_t h) {
-    uint32_t r0, r1;
-#if VGL_FMA_CARRY & 4
-    asm("{\n\t.reg .u32 c, e0, e1;\n\t.reg .b64 e;\n\t.reg .pred q;\n\t"
-        "mul.wide.u32 e, %4, %5;\n\t"          // e = h*EPS (FMA pipe)
-        "mov.b64 {e0, e1}, e;\n\t"
-        "add.cc.u32 %0, %2, e0;\n\t"
-        "addc.cc.u32 %1, %3, e1;\n\t"
-        "addc.u32 c, 0, 0;\n\t"
-        "mad.lo.cc.u32 %0, c, %5, %0;\n\t"     // += carry ? EPS : 0 (FMA pipe)
-        "madc.lo.u32 %1, c, %6, %1;\n\t"
-        "setp.eq.u32 q, %1, 0xffffffff;\n\t"
-        "setp.ne.and.u32 q, %0, 0, q;\n\t"
-        "@q mov.u32 %1, 0;\n\t"
-        "@q add.u32 %0, %0, 0xffffffff;\n\t}"
-        : "=&r"(r0), "=&r"(r1) : "r"(l0), "r"(l1), "r"(h), "r"(VGL_M1), "r"(VGL_ZERO));
-    return pack(r0, r1);
-#endif
-    asm("{\n\t.reg .u32 m, e0, e1;\n\t.reg .pred q;\n\t"
-        "sub.cc.u32 e0, 0, %4;\n\t"
-        "subc.u32 e1, %4, 0;\n\t"
-        "add.cc.u32 %0, %2, e0;\n\t"
-        "addc.cc.u32 %1, %3, e1;\n\t"
-        "addc.u32 m, 0, 0;\n\t"
-        "neg.s32 m, m;\n\t"
-        "add.cc.u32 %0, %0, m;\n\t"
-        "addc.u32 %1, %1, 0;\n\t"
-        "setp.eq.u32 q, %1, 0xffffffff;\n\t"
-        "setp.ne.and.u32 q, %0, 0, q;\n\t"
-        "@q mov.u32 %1, 0;\n\t"
-        "@q add.u32 %0, %0, 0xffffffff;\n\t}"
-        : "=&r"(r0), "=&r"(r1) : "r"(l0), "r"(l1), "r"(h));
-    return pack(r0, r1);
-}
-#endif
-
 // full 64x64 -> 128 product on 32-bit limbs (4 wide multiply-adds), then reduce
 __device__ __forceinline__ uint64_t mul(uint64_t a, uint64_t b) {
     const uint32_t a0 = (uint32_t)a, a1 = (uint32_t)(a >> 32), b0 = (uint32_t)b, b1 = (uint32_t)(b >> 32);
@@ -234,55 +199,6 @@ __device__ __forceinline__ uint64_t pow(uint64_t base, uint64_t e) {
         e >>= 1;
     }
     return r;
-}
-
-// x * 2^S mod p for a compile-time 0 <= S < 96 (x canonical -> canonical).
-// Every 2^k-th root of unity with k <= 6 is a power of two in this field
-// (2 has order 192), so radix-<=64 butterflies multiply by shifts only.
-// With phi = 2^32 (phi^2 = phi - 1, phi^3 = -1) and (l2:l1:l0) = x << (S mod 32):
-//   S <  32: (l1:l0) + l2*(2^32-1)
-//   S <  64: the general 128-bit reduction of (l2:l1:l0:0)
-//   S >= 64: l0*(2^32-1) - (l2:l1)
-// (Issuing the limb shifts as wide multiplies on the FMA pipe, or building the 64-bit sums from
-// mad.wide plus a 64-bit compare instead of carry chains, was measured slower on B200: radix-16
-// butterfly throughput 2004 and 1250 G element-stages/s against 2091 for this form.)
-template <int S>
-__device__ __forceinline__ uint64_t mul_pow2(uint64_t x) {
-    static_assert(S >= 0 && S < 96, "shift out of range");
-#ifdef __CUDA_ARCH__
-    if constexpr (S == 0) {
-        return x;
-    } else {
-        constexpr int V = S % 32, U = S / 32;
-        // (l2:l1:l0) = x << V as three 32-bit limbs
-        uint32_t l0 = (uint32_t)x, l1 = (uint32_t)(x >> 32), l2 = 0;
-        if constexpr (V != 0) {
-            l2 = l1 >> (32 - V); l1 = (l1 << V) | (l0 >> (32 - V)); l0 <<= V;
-        }
-        if constexpr (U == 0) {
-            // l0 + l1 phi + l2 phi^2 = (l1:l0) + l2*(2^32-1)
-            return add_mul_eps(l0, l1, l2);
-        } else if constexpr (U == 1) {
-            // l0 phi + l1 phi^2 + l2 phi^3: the 128-bit value (hi = (l2:l1), lo = (l0:0))
-            return reduce128(pack(0, l0), pack(l1, l2));
-        } else {
-            // l0 phi^2 + l1 phi^3 + l2 phi^4 = l0*(2^32-1) - (l2:l1); (l2:l1) < 2^63 is canonical
-#if VGL_FMA_CARRY & 4
-            uint64_t e;
-            asm("mul.wide.u32 %0, %1, %2;" : "=l"(e) : "r"(l0), "r"(VGL_M1));     // FMA pipe
-            return sub(e, pack(l1, l2));
-#else
-            uint32_t e0, e1;
-            asm("sub.cc.u32 %0, 0, %2;\n\t"
-                "subc.u32 %1, %2, 0;"
-                : "=&r"(e0), "=&r"(e1) : "r"(l0));
-            return sub(pack(e0, e1), pack(l1, l2));
-#endif
-        }
-    }
-#else
-    return x;
-#endif
 }
 
 // host-side helpers used when building twiddle tables
