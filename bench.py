@@ -537,8 +537,8 @@ def run_native(a):
                    "hash_columns": 8 * n}
         # DRAM bytes per message row from ncu captures of these kernels (dram read + write of one launch /
         # rows of that launch), valid for this geometry only; scaled to an average launch
-        ncu_per_row = {"encode_pass1": 1.597e6, "encode_mid": 2.515e6, "encode_pass3": 4.343e6,
-                       "hash_columns": 2.197e6} if (a.log_k, a.blowup) == (16, 4) else {}
+        ncu_per_row = {"encode_pass1": 0.938e6, "encode_mid": 2.484e6, "encode_pass3": 4.074e6,
+                       "hash_columns": 2.193e6} if (a.log_k, a.blowup) == (16, 4) else {}
         launches = sum(v[1] for v in prof.values())
         bytes_per_step = rows * per_row.get(dom[0], 0)
         dom_ms_per_step = dom[1][0] / a.steps

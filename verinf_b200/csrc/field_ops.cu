@@ -332,7 +332,8 @@ __global__ void __launch_bounds__(256) k_colsum_finish(const uint64_t* __restric
 // w = M.v: WPR warps of a CTA per row, lanes stride the row summing unreduced products, shuffle reduction.
 // Bound by reading M once; MATVEC_BATCH entries per lane are on the way at a time, and rows are shared between warps
 // until the GPU is full of them.  PAIRS: rows and v start on 16-byte boundaries and two entries come with a load.
-// 4096 x 11008: 89 us with one warp per row and a load at a time, 75 us so (4.8 TB/s).
+// 4096 x 11008, cold L2: 98 us with one warp per row and a load at a time, 81 us so (4.5 TB/s).  The matrix is read past L2
+// (evicted first); where it stays in L2 between calls (75 MB), rows of 1024 entries cost up to 15 % more than before.
 constexpr int MATVEC_BATCH = 8;
 template <int WPR, bool PAIRS>
 __global__ void __launch_bounds__(256) k_matvec(const uint64_t* __restrict__ M, const uint64_t* __restrict__ v,
@@ -382,7 +383,8 @@ __global__ void __launch_bounds__(256) k_matvec(const uint64_t* __restrict__ M, 
     }
     if (lane == 0 && row < m) w[row] = acc;
 }
-// Warps per row: doubled while all rows together leave room for them (64 warps per SM) and a warp keeps a whole batch.
+// Warps per row: doubled while all rows together need no more than 64 warps per SM (of which 48 are resident, at 40
+// registers) and a warp keeps a whole batch.
 int launch_matvec(const uint64_t* M, const uint64_t* v, uint64_t* w, int64_t m, int64_t n, cudaStream_t st) {
     int wpr = 1;
     while (wpr < 8 && m * wpr * 2 <= 148 * 64 && n >= wpr * 2 * 32 * MATVEC_BATCH) wpr *= 2;

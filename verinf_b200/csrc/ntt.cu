@@ -1080,9 +1080,9 @@ static int encode_impl(const uint64_t* msg, const KqSrc* kq, int64_t m, int64_t 
     VI_REQUIRE(scratch != nullptr && scratch_bytes >= per_row,
                "encode: scratch of at least %lld bytes required (see vi_encode_scratch_bytes)", (long long)per_row);
     int64_t chunk = scratch_bytes / per_row;
-    // Whole waves: with tiles per row a multiple of 16 (K >= 2^12) a row count that is a multiple of 37 makes
-    // every grid of the three passes a multiple of 148 SMs x 4 resident CTAs, so no launch ends in a
-    // nearly empty wave.
+    // A multiple of 37 = 148 / 4 rows: the last pass, 4 CTAs per SM, then ends in a full wave at K = 2^14 .. 2^16 and a
+    // blow-up of 4.  (us, 4096 x 2^16 / 5504 x 2^14 rows at a blow-up of 4: 12007 / 4945 so, 12089 / 4943 unrounded,
+    // 12060 / 4983 with rows that fill whole waves of all three passes at their own CTAs per SM.)
     if (chunk > 37 && chunk < m) chunk -= chunk % 37;
     const uint64_t *fs_inv, *fs_fwd = nullptr, *twist = nullptr;
     int rc = get_fs(k, n2, true, &fs_inv);        // inverse step 1: columns j2 (n2 of them), index k1

@@ -2,14 +2,15 @@
 //
 // What it replaces in the reference: prove_terms_gpu with fold_t and gl_sum (layergkr/gpu.py:326-410; CPU twin
 // layergkr/sumcheck.py:153-226).  sumcheck.cu keeps the per-round entry points whose samples stay on the device (for
-// sharded proofs); here the tables are read in place, the first fold writes the work buffer, and the last block of each
+// sharded proofs); here the tables are read in place (or copied as the first round of a session sums them), folds write the
+// work buffer, and the last block of each
 // round hands its sums to the host through mapped memory, so a round is one launch and no copy, and a queued proof waits
 // for the device once.
 //
 // What bounds it: large tables the integer pipes (a pair of entries costs 2 products per sample point), small ones the
 // chain of rounds.  Against both:
 //  * With the challenges known a kernel does two rounds per pass: it reads four entries per table and index, sums both
-//    rounds' polynomials and writes one entry.  A 3 x 2^24 proof moves 0.63 GB instead of 1.6 and is launched 8 times.
+//    rounds' polynomials and writes one entry.  A 3 x 2^24 proof moves 0.67 GB instead of 1.6 and is launched 8 times.
 //  * A round polynomial of degree d is summed at 0, infinity, -1 and 2 instead of 0..d: the value at infinity is the
 //    product of the differences, -1 is one subtraction away from 0, and the value at 1 follows from the round before.
 //    The host turns sums into coefficients and evaluates them (a few products per round).

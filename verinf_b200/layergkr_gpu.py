@@ -6,7 +6,8 @@ and return values): `encode_batch_ntt`, `hash_and_tree`, `prove_terms_gpu` on th
 
 `prove_terms_gpu` keeps the reference's per-round `coin` callback, but each round is one
 fused fold+evaluate launch that hands its sums to the host, instead of ~10 elementwise
-launches and a host sync per sample point, and the caller's tables are read where they are.
+launches and a host sync per sample point.  The caller's tables are read where they are; where a
+callback runs before the last read, a copy is kept.
 """
 import ctypes as C
 from typing import Callable, List, Optional, Sequence
